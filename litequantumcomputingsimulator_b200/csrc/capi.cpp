@@ -577,15 +577,17 @@ int lqcs_fusion_plan(uint32_t n_qubits, const lqcs_instruction* insts, uint64_t 
         const auto gates = lqcs_b200::decode_all(insts, n_insts, n_qubits);
         if (fusion_mode == lqcs_b200::kFuseTile) {
             // passes: width = number of high tile qubits, gates = gates applied by the pass
-            const auto items = lqcs_b200::plan_tiles(gates, n_qubits,
-                                                     lqcs_b200::default_tile_config(n_qubits));
+            const auto cfg = lqcs_b200::default_tile_config(n_qubits);
+            const auto form = lqcs_b200::uses_rotation_form(cfg)
+                                  ? lqcs_b200::rotation_form(gates, n_qubits) : gates;
+            const auto items = lqcs_b200::plan_tiles(form, n_qubits, cfg);
             *n_blocks = items.size();
             for (uint64_t i = 0; i < items.size() && i < cap; ++i) {
                 const bool pass = items[i].is_pass;
                 if (block_width)
                     block_width[i] = pass ? static_cast<uint32_t>(items[i].hbits.size())
-                                          : gates[items[i].gate].base_qubits();
-                if (block_gates) block_gates[i] = pass ? static_cast<uint32_t>(items[i].gates.size()) : 1;
+                                          : form[items[i].gate].base_qubits();
+                if (block_gates) block_gates[i] = lqcs_b200::source_gates(items[i], form);
             }
             return;
         }

@@ -182,6 +182,13 @@ void Program::launch_op(size_t i, const LaunchCtx& ctx, double2* st, uint32_t n,
             launch_pauli_rotation(ctx, st, n, batch, op.x, op.zy, op.n_y, op.cos_h, op.sin_h);
             break;
         case OpKind::TILE:
+            if (op.reg_tile && reg_passes[op.pass_index].rot) {
+                launch_rot_pass(ctx, st, n, batch, reg_passes[op.pass_index],
+                                reg_ops.data() + reg_op_off[op.pass_index],
+                                d_reg_layouts.as<RegLayout>() + reg_lay_off[op.pass_index],
+                                d_reg_mats.as<double2>() + reg_mat_off[op.pass_index]);
+                break;
+            }
             if (op.reg_tile) {
                 launch_reg_pass(ctx, st, n, batch, reg_passes[op.pass_index],
                                 d_reg_ops.as<RegOp>() + reg_op_off[op.pass_index],
@@ -238,19 +245,21 @@ static bool use_tiles(uint32_t n, const FusionConfig& fc) {
 }
 
 // Host side of a tile-pass program (ops not yet uploaded).
-static Program assemble_tiles(const std::vector<GateDesc>& gates, uint32_t n,
+static Program assemble_tiles(const std::vector<GateDesc>& source, uint32_t n,
                               const TileConfig& cfg, std::vector<DevOp>& ops) {
     Program p;
+    const std::vector<GateDesc> gates = uses_rotation_form(cfg) ? rotation_form(source, n) : source;
     for (const PlanItem& it : plan_tiles(gates, n, cfg)) {
         if (!it.is_pass) {
             ops.push_back(lower_gate(gates[it.gate], n));
+            ops.back().src_gates = source_gates(it, gates);
             continue;
         }
         DevOp op;
         op.kind = OpKind::TILE;
         op.k = static_cast<uint32_t>(it.hbits.size());
         op.targets = it.hbits;
-        op.src_gates = static_cast<uint32_t>(it.gates.size());
+        op.src_gates = source_gates(it, gates);
         op.alg_fraction = 1.0;
         if (cfg.reg) {
             RegPass rp;
@@ -271,7 +280,7 @@ static Program assemble_tiles(const std::vector<GateDesc>& gates, uint32_t n,
         // splits at each (the rotation runs on its own, the gates between as passes)
         auto smem_pass = [&](const PlanItem& part) {
             DevOp sop = op;
-            sop.src_gates = static_cast<uint32_t>(part.gates.size());
+            sop.src_gates = source_gates(part, gates);
             TilePass tp;
             p.pass_op_off.push_back(p.tile_ops.size());
             lower_pass(part, gates, cfg, tp, p.tile_ops, p.tile_mats, &sop.tile_flops);
@@ -289,6 +298,7 @@ static Program assemble_tiles(const std::vector<GateDesc>& gates, uint32_t n,
             if (!part.gates.empty()) smem_pass(part);
             part.gates.clear();
             ops.push_back(lower_gate(gates[gi], n));
+            ops.back().src_gates = gates[gi].src;
         }
         if (!part.gates.empty()) smem_pass(part);
     }
@@ -303,11 +313,12 @@ static std::vector<DevOp> dense_ops(const std::vector<GateDesc>& gates, uint32_t
     return lower_plan(plan(gates, n, g), gates, n);
 }
 
-bool compile_slots(const std::vector<GateDesc>& gates, uint32_t n,
+bool compile_slots(const std::vector<GateDesc>& source, uint32_t n,
                    const std::vector<std::vector<std::array<cd, 4>>>& slots, cudaStream_t stream,
                    Program& out) {
     if (n < kRegMinBits) return false;
     const TileConfig cfg = default_tile_config(n);
+    const std::vector<GateDesc> gates = uses_rotation_form(cfg) ? rotation_form(source, n) : source;
     Program p;
     std::vector<DevOp> ops;
     for (const PlanItem& it : plan_tiles(gates, n, cfg)) {
@@ -322,7 +333,7 @@ bool compile_slots(const std::vector<GateDesc>& gates, uint32_t n,
         op.kind = OpKind::TILE;
         op.k = static_cast<uint32_t>(it.hbits.size());
         op.targets = it.hbits;
-        op.src_gates = static_cast<uint32_t>(it.gates.size());
+        op.src_gates = source_gates(it, gates);
         op.alg_fraction = 1.0;
         op.reg_tile = true;
         RegPass rp;

@@ -55,8 +55,9 @@ double param(const GateDesc& g, size_t i) {
 
 // Apply a dense gate (matrix f on local positions pos[0..m-1] of a k-bit space) to a
 // small host vector v of 2^k entries.
-void apply_small(std::vector<cd>& v, uint32_t k, const std::vector<uint32_t>& pos,
-                 const std::vector<cd>& f) {
+// Products are formed in extended precision.
+void apply_small(std::vector<cl>& v, uint32_t k, const std::vector<uint32_t>& pos,
+                 const std::vector<cl>& f) {
     const uint32_t m = static_cast<uint32_t>(pos.size());
     const uint64_t dim = uint64_t{1} << m;
     std::vector<uint32_t> sorted = pos;
@@ -66,7 +67,7 @@ void apply_small(std::vector<cd>& v, uint32_t k, const std::vector<uint32_t>& po
         for (uint32_t j = 0; j < m; ++j)
             if ((l >> j) & 1) off[l] |= uint64_t{1} << pos[j];
     const uint64_t groups = (uint64_t{1} << k) >> m;
-    std::vector<cd> a(dim);
+    std::vector<cl> a(dim);
     for (uint64_t g = 0; g < groups; ++g) {
         uint64_t base = g;
         for (uint32_t p : sorted) {
@@ -75,8 +76,8 @@ void apply_small(std::vector<cd>& v, uint32_t k, const std::vector<uint32_t>& po
         }
         for (uint64_t l = 0; l < dim; ++l) a[l] = v[base | off[l]];
         for (uint64_t r = 0; r < dim; ++r) {
-            cd s{0.0, 0.0};
-            for (uint64_t c = 0; c < dim; ++c) s += f[r * dim + c] * a[c];
+            cl s{0.0, 0.0};
+            for (uint64_t c = 0; c < dim; ++c) s += wide_mul(f[r * dim + c], a[c]);
             v[base | off[r]] = s;
         }
     }
@@ -541,13 +542,13 @@ std::vector<FusedBlock> pack_consecutive(const std::vector<FusedBlock>& blocks,
     return out;
 }
 
-std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<GateDesc>& gates) {
+std::vector<cl> block_matrix_wide(const FusedBlock& b, const std::vector<GateDesc>& gates) {
     const uint32_t k = static_cast<uint32_t>(b.qubits.size());
     const uint64_t dim = uint64_t{1} << k;
-    std::vector<cd> m(dim * dim, cd{0, 0});
+    std::vector<cl> m(dim * dim, cl{0, 0});
     // columns evolve independently: column c starts as e_c
-    std::vector<std::vector<cd>> cols(dim, std::vector<cd>(dim, cd{0, 0}));
-    for (uint64_t c = 0; c < dim; ++c) cols[c][c] = 1.0;
+    std::vector<std::vector<cl>> cols(dim, std::vector<cl>(dim, cl{0, 0}));
+    for (uint64_t c = 0; c < dim; ++c) cols[c][c] = 1.0L;
     for (uint32_t gi : b.gates) {
         const GateDesc& g = gates[gi];
         std::vector<uint32_t> pos;
@@ -555,11 +556,22 @@ std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<GateDesc>& g
             const auto it = std::find(b.qubits.begin(), b.qubits.end(), q);
             pos.push_back(static_cast<uint32_t>(it - b.qubits.begin()));
         }
-        const std::vector<cd> f = g.full_matrix();
+        std::vector<cl> f;
+        if (g.n_controls == 0 && !g.wide.empty()) {
+            f = g.wide;
+        } else {
+            for (const cd& z : g.full_matrix()) f.push_back(z);
+        }
         for (uint64_t c = 0; c < dim; ++c) apply_small(cols[c], k, pos, f);
     }
     for (uint64_t c = 0; c < dim; ++c)
         for (uint64_t r = 0; r < dim; ++r) m[r * dim + c] = cols[c][r];
+    return m;
+}
+
+std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<GateDesc>& gates) {
+    std::vector<cd> m;
+    for (const cl& z : block_matrix_wide(b, gates)) m.push_back(narrow(z));
     return m;
 }
 

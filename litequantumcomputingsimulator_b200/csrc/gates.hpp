@@ -14,6 +14,12 @@
 namespace lqcs_b200 {
 
 using cd = std::complex<double>;
+// Products of gate matrices are formed in extended precision and rounded once.
+using cl = std::complex<long double>;
+inline cl wide_mul(const cl& a, const cl& b) {
+    return {a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()};
+}
+inline cd narrow(const cl& z) { return {static_cast<double>(z.real()), static_cast<double>(z.imag())}; }
 
 // Error carrying one of the lqcs_status codes; the C ABI turns it into a status code and
 // the message returned by lqcs_last_error().
@@ -42,6 +48,8 @@ struct GateDesc {
     // as a phase, diagonal or X.
     bool slot = false;
     uint32_t slot_id = 0;
+    uint32_t src = 1;                    // source gates this one stands for (rotation_form)
+    std::vector<cl> wide;                // base_matrix before rounding, where known
 
     uint32_t base_qubits() const;        // Gate::base_qubits (src/circuit/gate.cpp:27-49)
     bool is_unitary() const;             // not Measure / Reset / Barrier / Kraus
@@ -134,6 +142,7 @@ std::vector<FusedBlock> pack_consecutive(const std::vector<FusedBlock>& blocks,
                                          uint32_t max_width);
 
 // Dense matrix of a block (block-local bit j <-> qubits[j]).
+std::vector<cl> block_matrix_wide(const FusedBlock& b, const std::vector<GateDesc>& gates);
 std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<GateDesc>& gates);
 
 // Turn a plan into device ops (single-gate blocks keep their specialised kernel).

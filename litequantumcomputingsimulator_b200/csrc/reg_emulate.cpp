@@ -19,6 +19,7 @@
 // The emulation follows reg_tile_kernels.cu line for line in what it computes; its
 // arithmetic is plain std::complex<double> (results agree with the device within rounding).
 #include <algorithm>
+#include <bit>
 #include <complex>
 #include <cstring>
 #include <sstream>
@@ -297,11 +298,12 @@ void emulate_reg_pass(const RegPass& pass, const RegOp* ops, const RegLayout* la
                         for (uint32_t q = 0; q < op.nterm; ++q) {
                             const cd meta = term[2 * q + 1];
                             const uint64_t hi = static_cast<uint64_t>(meta.imag());
-                            const uint64_t gc = static_cast<uint64_t>(meta.real()) | ((hi >> 6) << 32);
-                            const uint32_t em = static_cast<uint32_t>(hi & 63u);
-                            if ((base & gc) == gc && (e & em) == em) acc = term[2 * q] * acc;
+                            const uint64_t gc = static_cast<uint64_t>(meta.real()) | ((hi >> 12) << 32);
+                            const uint32_t bits = static_cast<uint32_t>(hi & 63u),
+                                           value = static_cast<uint32_t>((hi >> 6) & 63u);
+                            if ((base & gc) == gc && (e & bits) == value) acc = term[2 * q] * acc;
                         }
-                        const size_t at = dyn_base + op.dyn_off + e;
+                        const size_t at = dyn_base + (op.kind == kRegStage ? op.dyn_table : op.dyn_off) + e;
                         model.access(dyn_base_slot + at, t, true, "per-tile table write", log, tid, pass_index);
                         dyn[at] = acc;
                     }
@@ -345,7 +347,7 @@ void emulate_reg_pass(const RegPass& pass, const RegOp* ops, const RegLayout* la
                     cd* vt = &v[t * kE];
                     for (uint32_t i = o; i < end; ++i) {
                         const RegOp& op = ops[i];
-                        if ((base & op.gcmask) != op.gcmask) continue;
+                        if (op.kind != kRegStage && (base & op.gcmask) != op.gcmask) continue;
                         if (op.kind == kRegPauli) {   // rcmask / tcmask: Z-type bits
                             if (!in) continue;
                             const cd c = mats[op.mat_off];
@@ -371,6 +373,60 @@ void emulate_reg_pass(const RegPass& pass, const RegOp* ops, const RegLayout* la
                                 vt[u] = c * a + sign(u) * y * b;
                                 vt[w] = c * b + sign(w) * y * a;
                             }
+                            continue;
+                        }
+                        auto mask = [&](uint32_t at) {
+                            return std::bit_cast<uint64_t>(mats[at].real());
+                        };
+                        auto odd = [&](uint64_t mk) { return (__builtin_popcountll(base & mk) & 1) != 0; };
+                        if (op.kind == kRegStage) {
+                            uint32_t e0 = 0;
+                            for (uint32_t j = 0; j < kRegMaxDiag; ++j) e0 |= ((t >> op.loc[j]) & 1u) << j;
+                            const uint32_t off[kRegBits] = {op.nsel, op.selq[0], op.selq[1], op.rcmask};
+                            for (uint32_t u = 0; op.pad && u < kE; ++u) {
+                                uint32_t e = e0;
+                                for (uint32_t i2 = 0; i2 < kRegBits; ++i2)
+                                    if ((u >> i2) & 1u) e += off[i2];
+                                cd f;
+                                if (op.nterm) {
+                                    const size_t at = dyn_base + op.dyn_table + e;
+                                    model.access(dyn_base_slot + at, t, false, "per-tile table read", log,
+                                                 tid, pass_index);
+                                    f = dyn[at];
+                                } else {
+                                    f = mats[op.mat_off + e];
+                                }
+                                if (in) vt[u] *= f;
+                            }
+                            if (!in) continue;
+                            const uint32_t nr = static_cast<uint32_t>(__builtin_popcount(op.code));
+                            uint32_t j = 0;
+                            for (uint32_t c = op.code; c; c &= c - 1, ++j) {
+                                const uint32_t TM = c & (0u - c);
+                                const bool neg = op.tcmask < kRegSignBits
+                                                     ? odd(mask(p.sign_off + op.tcmask + j))
+                                                     : op.tcmask > kRegSignBits && odd(mask(op.dyn_off + nr + j));
+                                const cd xy = (neg ? -1.0 : 1.0) * mats[op.dyn_off + j];
+                                for (uint32_t b = 0; b < kE; ++b) {
+                                    if (b & TM) continue;
+                                    vt[b] += xy.real() * vt[b | TM];
+                                    vt[b | TM] += xy.imag() * vt[b];
+                                }
+                            }
+                            continue;
+                        }
+                        if (op.kind == kRegSign) {
+                            if (!in) continue;
+                            uint32_t z = 0;
+                            for (uint32_t j = 0; j < op.nterm; ++j) {
+                                const uint64_t mk = mask(op.mat_off + j);
+                                if (j <= m ? odd(mk) : (base & mk) == mk) z |= 1u << j;
+                            }
+                            const uint32_t whole = static_cast<uint32_t>(__builtin_popcount(z >> m));
+                            for (uint32_t u = 0; u < kE; ++u)
+                                if ((__builtin_popcount(t & z) + __builtin_popcount(u & (z >> kTB) & (kE - 1)) +
+                                     whole) & 1)
+                                    vt[u] = -vt[u];
                             continue;
                         }
                         if ((t & op.tcmask) != op.tcmask) continue;
@@ -540,9 +596,10 @@ void emulate_reg_pass(const RegPass& pass, const RegOp* ops, const RegLayout* la
             if (in) {
                 for (uint32_t t = 0; t < kT; ++t) {
                     const RegLayout& ly = lays[cur[t]];
+                    const uint64_t undo = p.rot ? std::bit_cast<uint64_t>(mats[0].real()) : 0;
                     const uint64_t g = base | thread_goff(ly, kTB, sgbit, t);
                     for (uint32_t u = 0; u < kE; ++u) {
-                        const uint64_t a = g | reg_goff(ly, sgbit, u);
+                        const uint64_t a = (g | reg_goff(ly, sgbit, u)) ^ undo;
                         out[a] = v[t * kE + u];
                         if (amps) {
                             ++amps->written[a];
@@ -580,8 +637,9 @@ void emulate_register_program(uint32_t n, const lqcs_instruction* insts, uint64_
                               uint64_t grid, int sync_tiles, bool pipe, bool drop_load_barrier,
                               cd* state, uint64_t race_ctas, uint64_t* n_passes,
                               uint64_t* n_races, std::string* report) {
-    const auto gates = decode_all(insts, n_insts, n);
     const TileConfig cfg = default_tile_config(n);
+    auto gates = decode_all(insts, n_insts, n);
+    if (uses_rotation_form(cfg)) gates = rotation_form(gates, n);
     if (!cfg.reg) invalid("register tile emulation: register passes are switched off");
     const auto items = plan_tiles(gates, n, cfg);
     RaceLog log;

@@ -19,7 +19,8 @@ constexpr size_t kTileMaxSmem = 200 * 1024;      // tile + staged operation reco
 
 // kTilePauli: a Pauli rotation exp(-i theta/2 P) inside a register pass (planner only; the
 // shared-memory kernel has no such operation).
-enum : uint8_t { kTileDense = 0, kTileDiag = 1, kTilePhase = 2, kTilePauli = 3 };
+// kTileRot: a real one-qubit map [[1, x], [y, 1]] (register passes in rotation form).
+enum : uint8_t { kTileDense = 0, kTileDiag = 1, kTilePhase = 2, kTilePauli = 3, kTileRot = 4 };
 
 // Shared-memory slot of tile element i: the low 3 bits are XOR-ed with a fold of the
 // higher bits so that power-of-two strides spread over the 8 16-byte positions of a
@@ -108,8 +109,25 @@ constexpr uint32_t kRegPauliMaxFlips = 9;       // X/Y qubits of a Pauli rotatio
 // mask) or lanes (loc[0] = their lane mask: the partner comes by shuffle), its Z-type bits zy
 // are register bits (rcmask), thread bits (tcmask) or out-of-tile qubits (a 64-bit mask among
 // its matrices: (cos, 0), y, then the mask as two exact 32-bit halves).
+//
+// Passes in rotation form (RegPass::rot, reg_rot_kernels.cu) have four more:
+// kRegStage: an optional diagonal table, then rotations.  The table (pad = 1) covers k tile
+// bits; entry bit j is thread bit loc[j] (31: none), register bit i adds the entry offset nsel,
+// selq[0], selq[1], rcmask (i = 0..3; 0 if the table does not use it); with nterm gated terms it
+// is built per tile (at dyn_table among the per-tile tables) like kRegDiagDyn's.  A rotation is
+// a0 += x a1, then a1 += y a0 with real x, y, on each register bit of `code`: what is left of a
+// one-qubit gate once its diagonal factors have moved into the neighbouring tables; their (x, y)
+// are at dyn_off among the matrices, bits ascending.  tcmask: the index of their signs (of x and
+// y; a Z on the bit that has moved past the rotation) in the tile's sign bits; kRegSignBits:
+// none; above: the masks of outside qubits follow the factors.  Sign bit j of a tile is the
+// parity of its index on mask j of the n_signs masks at sign_off.  The pass's first matrix entry
+// is the pattern of the qubits whose bits the store negates.
+// kRegSign: amplitude signs.  nterm masks: per thread-index bit, then per register bit, the
+// outside qubits whose parity puts a Z on it; then those whose parity negates the tile; then,
+// per mask, those that negate it where they are all 1.
 enum : uint8_t { kRegDense = 0, kRegDiag = 1, kRegPhase = 2, kRegSwapX = 3, kRegRemap = 4,
-                 kRegDiagDyn = 5, kRegMma = 6, kRegPauli = 7 };
+                 kRegDiagDyn = 5, kRegMma = 6, kRegPauli = 7, kRegStage = 8, kRegSign = 9 };
+constexpr uint32_t kRegSignBits = 60;   // sign bits of a tile (64-bit word, the top ones 0)
 
 struct RegLayout {
     uint16_t rsw[kRegBits];   // tile_swizzle(1 << rpos[i])
@@ -119,21 +137,25 @@ struct RegLayout {
     uint8_t pad[1];
 };
 
-struct RegOp {
-    uint64_t gcmask;          // qubits outside the tile that must all be 1
+struct alignas(16) RegOp {
+    union {
+        uint64_t gcmask;      // qubits outside the tile that must all be 1
+        uint16_t dyn_table;   // stage: first entry of its per-tile table
+    };
     uint32_t mat_off;         // double2 offset in the pass's staged matrices
     uint8_t kind;
-    uint8_t code;             // dense / swap: register target mask; remap: new layout index
-    uint8_t k;                // dense / diag: number of targets; remap: 1 = warp-local
+    uint8_t code;             // dense / swap / stage: register target mask; remap: new layout
+    uint8_t k;                // dense / diag / stage: number of targets; remap: 1 = warp-local
     uint8_t rcmask;           // register-index bits that must be 1 (controls, phase bits)
     uint16_t tcmask;          // thread-index bits that must be 1
     uint8_t loc[kRegMaxDiag]; // diag: target j at register bit loc, or thread bit loc & 0x7f
                               // when loc & 0x80
     uint8_t nsel;             // dense / diag: the tile's bits at qubits selq[0..nsel) pick
     uint8_t selq[kRegMaxSelect];   // one of 2^nsel consecutive matrices
-    uint8_t nterm;            // per-tile diagonal: gated phase terms
+    uint8_t nterm;            // per-tile diagonal: gated phase terms; rotation, sign: see above
     uint16_t dyn_off;         // per-tile diagonal: first entry in the per-tile tables
-    uint8_t pad[2];
+    uint8_t pad;              // stage: has a table
+    uint8_t pad2;
 };
 
 struct RegPass {
@@ -152,7 +174,11 @@ struct RegPass {
     uint8_t store_qubit[kRegMaxBits];   // of qubit store_qubit[b]
     uint32_t load_barrier;    // a barrier between the tile's loads and stores is needed and no
                               // other barrier provides it (relabelled stores, in place)
-    uint32_t fma_dense;       // some record is a dense op on register bits (kRegDense)
+    uint32_t last_layout;     // the layout the tile is stored from
+    uint32_t rot;             // rotation form (reg_rot_kernels.cu)
+    uint32_t n_signs, sign_off;
+    uint32_t fma_dense;       // some record is a dense op on register bits (kRegDense; rotation
+                              // form: or an unmerged diagonal)
     uint32_t mma_ops;         // some record is a tensor-path block (kRegMma)
     uint32_t pauli_ops;       // some record is a Pauli rotation (kRegPauli)
 };
@@ -162,6 +188,12 @@ static_assert(sizeof(RegLayout) % 4 == 0 && sizeof(RegOp) == 32, "staged as 32-b
 void launch_reg_pass(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t batch,
                      const RegPass& pass, const RegOp* d_ops, const RegLayout* d_layouts,
                      const double2* d_mats);
+// ops: the pass's records in host memory (a kernel parameter).
+void launch_rot_pass(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t batch,
+                     const RegPass& pass, const RegOp* ops, const RegLayout* d_layouts,
+                     const double2* d_mats);
+// LQCS_REG_PIPE: the double-buffered kernel, which runs passes of dense operations.
+bool reg_pipe_enabled();
 // Shared memory of a register pass holding `tiles` tile buffers (2: double-buffered kernel).
 size_t reg_smem_bytes(const RegPass& pass, uint32_t tiles = 1);
 constexpr size_t kRegPipeMaxSmem = 220 * 1024;   // double-buffered kernel, one CTA per SM at m = 12

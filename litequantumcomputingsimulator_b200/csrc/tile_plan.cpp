@@ -8,8 +8,10 @@
 // or select the amplitudes a phase multiplies).  Inside a pass, neighbouring gates on tile
 // qubits are fused into dense operations of at most `inner` qubits.
 #include <algorithm>
+#include <bit>
 #include <cmath>
 #include <cstdlib>
+#include <deque>
 #include <tuple>
 
 #include "tile_plan.hpp"
@@ -76,6 +78,195 @@ static bool tile_requirements(const GateDesc& g, const TileConfig& c, std::vecto
     for (uint32_t j = 0; j < k; ++j) need.push_back(g.targets()[j]);
     (void)c;
     return true;
+}
+
+namespace {
+
+bool is_x_matrix(const std::vector<cd>& m) {
+    return m.size() == 4 && m[0] == cd{0, 0} && m[1] == cd{1, 0} && m[2] == cd{1, 0} &&
+           m[3] == cd{0, 0};
+}
+
+// An uncontrolled one-qubit gate with a matrix of its own.
+bool plain_1q(const GateDesc& g) {
+    return g.is_unitary() && g.n_controls == 0 && g.type != LQCS_GATE_PAULI_ROTATION &&
+           g.type != LQCS_GATE_PERMUTATION && g.type != LQCS_GATE_SWAP && g.base_qubits() == 1;
+}
+
+GateDesc simple_gate(int type, std::vector<uint32_t> qubits, uint32_t n_controls,
+                     std::vector<double> params = {}) {
+    GateDesc g;
+    g.type = type;
+    g.qubits = std::move(qubits);
+    g.n_controls = n_controls;
+    g.params = std::move(params);
+    return g;
+}
+
+}  // namespace
+
+std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t n) {
+    using M2 = std::array<cl, 4>;
+    // What each gate is to its neighbours on a qubit: an X with controls (on its target), a
+    // one-qubit gate that is (not) diagonal, a dense two-qubit gate that takes one-qubit
+    // factors for free, or anything else.
+    enum Role : uint8_t { kOther, kCtrlX, kDiag1, kDense1, kDense2 };
+    std::vector<Role> role(gates.size(), kOther);
+    std::vector<std::vector<uint32_t>> on(n);   // gates touching each qubit, in order
+    std::vector<uint32_t> at(gates.size(), 0);  // index of gate i in its target's list
+    for (uint32_t i = 0; i < gates.size(); ++i) {
+        const GateDesc& g = gates[i];
+        if (g.type == LQCS_GATE_BARRIER) {
+            for (auto& v : on) v.push_back(i);
+            continue;
+        }
+        if (g.slot) {
+            role[i] = kDense1;
+        } else if (g.is_unitary() && g.type != LQCS_GATE_PAULI_ROTATION &&
+                   g.type != LQCS_GATE_PERMUTATION) {
+            if (g.base_qubits() == 1) {
+                const std::vector<cd> m = g.base_matrix();
+                if (g.n_controls == 0)
+                    role[i] = m[1] == cd{0, 0} && m[2] == cd{0, 0} ? kDiag1 : kDense1;
+                else if (is_x_matrix(m) && g.qubits.size() <= 8)
+                    role[i] = kCtrlX;
+            } else if (g.base_qubits() == 2 && g.n_controls == 0 && g.type != LQCS_GATE_RZZ &&
+                       g.type != LQCS_GATE_SWAP) {
+                role[i] = kDense2;
+            }
+        }
+        if (role[i] == kCtrlX) at[i] = static_cast<uint32_t>(on[g.targets()[0]].size());
+        for (uint32_t q : g.qubits) on[q].push_back(i);
+    }
+    // the neighbour of gate i on its target in direction dir takes the H (diagonal one-qubit
+    // gates in between merge with it)
+    auto absorbs = [&](uint32_t i, int dir) {
+        const uint32_t t = gates[i].targets()[0];
+        const std::vector<uint32_t>& v = on[t];
+        for (int64_t k = static_cast<int64_t>(at[i]) + dir;
+             k >= 0 && k < static_cast<int64_t>(v.size()); k += dir) {
+            const uint32_t j = v[static_cast<size_t>(k)];
+            if (role[j] == kDiag1) continue;
+            return role[j] == kDense1 || role[j] == kDense2 ||
+                   (role[j] == kCtrlX && gates[j].targets()[0] == t);
+        }
+        return false;
+    };
+
+    std::vector<GateDesc> out;
+    uint32_t carry = 0;   // source gates of products that turned out to be the identity
+    struct Pending {
+        M2 m{};
+        uint32_t count = 0, src = 0;
+        GateDesc one;   // the gate itself while it is the only one
+    };
+    std::vector<Pending> pend(n);
+    auto push = [&](GateDesc g) {
+        g.src += carry;
+        carry = 0;
+        out.push_back(std::move(g));
+    };
+    auto multiply = [&](uint32_t q, const GateDesc& g, uint32_t src) {
+        Pending& p = pend[q];
+        std::vector<cl> a = g.wide;
+        if (a.empty())
+            for (const cd& z : g.base_matrix()) a.push_back(z);
+        if (p.count == 0) {
+            p.m = {a[0], a[1], a[2], a[3]};
+            p.one = g;
+        } else {
+            const M2 b = p.m;
+            p.m = {wide_mul(a[0], b[0]) + wide_mul(a[1], b[2]),
+                   wide_mul(a[0], b[1]) + wide_mul(a[1], b[3]),
+                   wide_mul(a[2], b[0]) + wide_mul(a[3], b[2]),
+                   wide_mul(a[2], b[1]) + wide_mul(a[3], b[3])};
+        }
+        ++p.count;
+        p.src += src;
+    };
+    auto flush = [&](uint32_t q) {
+        Pending& p = pend[q];
+        if (p.count == 0) return;
+        constexpr long double tol = 5e-16L;
+        if (p.count > 1 && std::abs(p.m[0] - cl{1, 0}) < tol && std::abs(p.m[1]) < tol &&
+            std::abs(p.m[2]) < tol && std::abs(p.m[3] - cl{1, 0}) < tol) {
+            carry += p.src;   // such as the H H between two exchanged X
+        } else {
+            GateDesc g;
+            if (p.count == 1) {
+                g = std::move(p.one);
+            } else {
+                g = simple_gate(LQCS_GATE_UNITARY, {q}, 0);
+                for (const cl& z : p.m) g.mat.push_back(narrow(z));
+                g.wide.assign(p.m.begin(), p.m.end());
+            }
+            g.src = p.src;
+            push(std::move(g));
+        }
+        p = Pending{};
+    };
+    for (uint32_t i = 0; i < gates.size(); ++i) {
+        const GateDesc& g = gates[i];
+        if (g.type == LQCS_GATE_BARRIER) {
+            for (uint32_t q = 0; q < n; ++q) flush(q);
+            push(g);
+            continue;
+        }
+        if (!g.slot && plain_1q(g)) {
+            multiply(g.qubits[0], g, g.src);
+            continue;
+        }
+        if (role[i] == kCtrlX && (absorbs(i, -1) || absorbs(i, 1))) {
+            const uint32_t t = g.targets()[0];
+            // The H before rounds 1/sqrt(2) up and the H after rounds it down: two of the same
+            // would scale the state by 1 + 2e-16 for every exchanged X where they are folded
+            // into dense blocks.
+            GateDesc h = simple_gate(LQCS_GATE_UNITARY, {t}, 0);
+            const long double r = std::sqrt(0.5L);
+            h.wide = {r, r, r, -r};
+            auto rounded = [&](double x) { h.mat = {x, x, x, -x}; };
+            const double nearest = static_cast<double>(r);
+            rounded(nearest);
+            multiply(t, h, 0);
+            for (uint32_t q : g.qubits) flush(q);
+            GateDesc z = simple_gate(LQCS_GATE_Z, g.qubits, g.n_controls);
+            z.src = g.src;
+            push(std::move(z));
+            rounded(std::nextafter(nearest, nearest > r ? 0.0 : 1.0));
+            multiply(t, h, 0);
+            continue;
+        }
+        if (g.type == LQCS_GATE_RZZ && g.n_controls == 0) {
+            // diag(e^-i, e^i, e^i, e^-i)(theta/2): RZ(theta) on a, P(theta) on b, CP(-2 theta);
+            // the one-qubit factors join a pending product, or wait for the next gate
+            const uint32_t a = g.qubits[0], b = g.qubits[1];
+            const double th = g.params.at(0);
+            const uint32_t rz = pend[b].count > 0 && pend[a].count == 0 ? b : a;
+            const uint32_t ph = rz == a ? b : a;
+            GateDesc grz = simple_gate(LQCS_GATE_RZ, {rz}, 0, {th});
+            GateDesc gph = simple_gate(LQCS_GATE_P, {ph}, 0, {th});
+            auto unit = [](long double x) { return cl{std::cos(x), std::sin(x)}; };
+            grz.wide = {unit(-0.5L * th), 0.0L, 0.0L, unit(0.5L * th)};
+            gph.wide = {1.0L, 0.0L, 0.0L, unit(th)};
+            const bool rz_now = pend[rz].count > 0, ph_now = pend[ph].count > 0;
+            if (rz_now) multiply(rz, grz, 0);
+            if (ph_now) multiply(ph, gph, 0);
+            flush(a);
+            flush(b);
+            GateDesc cp = simple_gate(LQCS_GATE_P, {a, b}, 1, {-2.0 * th});
+            cp.src = g.src;
+            cp.wide = {1.0L, 0.0L, 0.0L, unit(-2.0L * th)};
+            push(std::move(cp));
+            if (!rz_now) multiply(rz, grz, 0);
+            if (!ph_now) multiply(ph, gph, 0);
+            continue;
+        }
+        for (uint32_t q : g.qubits) flush(q);
+        push(g);
+    }
+    for (uint32_t q = 0; q < n; ++q) flush(q);
+    if (carry && !out.empty()) out.back().src += carry;
+    return out;
 }
 
 // First-fit picks the high tile qubits in the order gates ask for them, which is often not
@@ -315,18 +506,14 @@ void set_groups(TileOp& op, std::vector<uint32_t> pos, uint32_t lcmask, uint32_t
         op.dhi[j] = static_cast<uint16_t>(tile_swizzle(deposit(j * kTileThreads, pos) | lcmask));
 }
 
-bool is_x(const std::vector<cd>& m) {
-    return m.size() == 4 && m[0] == cd{0, 0} && m[1] == cd{1, 0} && m[2] == cd{1, 0} &&
-           m[3] == cd{0, 0};
-}
-
 }  // namespace
 
 double local_op_flops(const LocalOp& o, bool x_free) {
     if (o.kind == kTilePauli) return o.lt.empty() ? 6.0 : 16.0;   // op_flops_per_amp of PAULI
+    if (o.kind == kTileRot) return 4.0;
     const double frac = std::ldexp(1.0, -(__builtin_popcount(o.lmask) + __builtin_popcountll(o.gcmask)));
     if (o.kind != kTileDense) return 6.0 * frac;
-    if (x_free && !o.variant && o.lt.size() == 1 && o.sel.empty() && is_x(o.m)) return 0.0;
+    if (x_free && !o.variant && o.lt.size() == 1 && o.sel.empty() && is_x_matrix(o.m)) return 0.0;
     return 8.0 * std::ldexp(1.0, static_cast<int>(o.lt.size())) * frac;
 }
 
@@ -358,23 +545,24 @@ static void fold_into(LocalOp& q, const LocalOp& p, uint32_t j, const std::vecto
         }
         for (uint64_t r = 0; r < D; ++r) {
             for (uint64_t c = 0; c < D; ++c) {
-                cd acc{0, 0};
+                cl acc{0, 0};
                 if (after) {
                     // (U M)[r][c] = sum_x U[r_j][x] M[r with bit j = x][c]
                     const uint64_t rj = (r >> j) & 1, r0 = r & ~(uint64_t{1} << j);
                     for (uint64_t xj = 0; xj < 2; ++xj)
-                        acc += u[rj * 2 + xj] * m[(r0 | xj << j) * D + c];
+                        acc += wide_mul(u[rj * 2 + xj], m[(r0 | xj << j) * D + c]);
                 } else {
                     // (M U)[r][c] = sum_x M[r][x] U[x][c]; U acts on bit j only
                     const uint64_t cj = (c >> j) & 1, c0 = c & ~(uint64_t{1} << j);
                     for (uint64_t xj = 0; xj < 2; ++xj)
-                        acc += m[r * D + (c0 | xj << j)] * u[xj * 2 + cj];
+                        acc += wide_mul(m[r * D + (c0 | xj << j)], u[xj * 2 + cj]);
                 }
-                out.push_back(acc);
+                out.push_back(narrow(acc));
             }
         }
     }
     q.m = std::move(out);
+    q.wide.clear();
     q.sel = sel;
 }
 
@@ -597,11 +785,83 @@ static void fold_single_qubit_ops(std::vector<LocalOp>& ops, uint32_t max_select
     ops.resize(w);
 }
 
+// M = diag(l0, l1) L diag(1, r1) E with L = [[1, x], [y, 1 + x y]] (a0 += x a1, then
+// a1 += y a0) and real x, y; E: the exchange of the two halves where `exchange`, else the
+// identity.  Every unitary has this form with |x| <= 1, |y| <= 1/2: up to row scales L is then a
+// rotation by at most 45 degrees, so the two FMAs round like one, and L needs no register
+// besides the pair.  Real matrices and some others have it too; false for the rest.  l0 and l1
+// carry the row norms that rounding x and y would change (a drift of the state's norm, which
+// would add up over the gates).
+static bool rotation_split(const LocalOp& o, bool& exchange, cl& r1, double& x, double& y, cl& l0,
+                           cl& l1) {
+    auto entry = [&](int e) { return o.wide.empty() ? cl{o.m[e]} : o.wide[e]; };
+    cl a = entry(0), b = entry(1), c = entry(2), d = entry(3);
+    exchange = std::max(std::abs(b), std::abs(c)) > std::max(std::abs(a), std::abs(d));
+    if (exchange) {
+        std::swap(a, b);
+        std::swap(c, d);
+    }
+    const long double ad = std::min(std::abs(a), std::abs(d));
+    if (!(ad > 0.0L) || !(std::max(std::abs(b), std::abs(c)) <= 1.001L * ad)) return false;
+    l0 = a;
+    l1 = d;
+    r1 = 1.0L;
+    x = y = 0.0;
+    if (b == cl{0, 0} && c == cl{0, 0}) return true;
+    const cl via_b = b / a, via_c = c / d;   // X r1 and Y / r1 of the rows (1, X), (Y, 1)
+    r1 = std::abs(via_b) >= std::abs(via_c) ? via_b / std::abs(via_b)
+                                            : std::conj(via_c) / std::abs(via_c);
+    const cl xc = wide_mul(via_b, std::conj(r1)), yc = wide_mul(via_c, r1);
+    if (std::abs(xc.imag()) > 1e-15L || std::abs(yc.imag()) > 1e-15L) return false;
+    const long double X = xc.real(), Y = yc.real(), det = 1.0L - X * Y;
+    if (det < 0.25L) return false;   // nearly singular
+    x = static_cast<double>(X);
+    y = static_cast<double>(Y / det);
+    const long double s1 = 1.0L + static_cast<long double>(x) * y;
+    l0 *= std::sqrt((1.0L + X * X) / (1.0L + static_cast<long double>(x) * x));
+    l1 = wide_mul(d, std::conj(r1)) * std::sqrt((1.0L + Y * Y) / (static_cast<long double>(y) * y + s1 * s1));
+    return true;
+}
+
+// Uncontrolled one-qubit dense operations as diagonal, real rotation, diagonal.  One whose
+// matrix differs per state keeps the same three operations for every state.
+static void split_rotations(std::vector<LocalOp>& ops) {
+    std::vector<LocalOp> out;
+    out.reserve(2 * ops.size());
+    const cl one{1, 0};
+    for (LocalOp& o : ops) {
+        bool ex = false;
+        cl r1, l0, l1;
+        double x = 0, y = 0;
+        if (o.kind != kTileDense || o.lt.size() != 1 || o.lmask || o.gcmask || !o.sel.empty() ||
+            (!o.variant && is_x_matrix(o.m)) || !rotation_split(o, ex, r1, x, y, l0, l1)) {
+            out.push_back(std::move(o));
+            continue;
+        }
+        LocalOp before, rot, after;
+        before.kind = after.kind = kTileDiag;
+        rot.kind = kTileRot;
+        before.lt = rot.lt = after.lt = o.lt;
+        before.variant = rot.variant = after.variant = o.variant;
+        // diag(1, r1) E = E diag(r1, 1)
+        before.wide = ex ? std::vector<cl>{r1, one} : std::vector<cl>{one, r1};
+        rot.m = {cd{x, y}};
+        rot.exchange = ex;
+        after.wide = {l0, l1};
+        for (LocalOp* d : {&before, &after}) d->m = {narrow(d->wide[0]), narrow(d->wide[1])};
+        if (o.variant || r1 != one) out.push_back(std::move(before));
+        out.push_back(std::move(rot));
+        if (o.variant || l0 != one || l1 != one) out.push_back(std::move(after));
+    }
+    ops = std::move(out);
+}
+
 std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<GateDesc>& gates,
                                     const TileConfig& cfg, uint32_t max_select,
                                     const std::vector<std::array<cd, 4>>* slot_mats,
                                     uint32_t max_diag, bool dyn_terms,
-                                    std::vector<uint32_t>* store_qubits, bool native_rotations) {
+                                    std::vector<uint32_t>* store_qubits, bool native_rotations,
+                                    bool rot) {
     LocalMap lm{cfg.L, item.hbits, {}};
     std::vector<LocalOp> out;
     // a noise slot takes this state's matrix (identity when no table is given)
@@ -636,6 +896,7 @@ std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<Gate
                 else op.gcmask |= uint64_t{1} << q;
             }
             op.m.push_back(g.base_matrix()[3]);
+            if (!g.wide.empty()) op.wide = {g.wide[3]};
             out.push_back(std::move(op));
             return;
         }
@@ -651,6 +912,11 @@ std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<Gate
             else gc |= uint64_t{1} << q;
         }
         out.push_back(matrix_op(resolved(g).base_matrix(), lt, lc, gc, g.slot));
+        if (g.wide.size() == 4) {
+            LocalOp& op = out.back();
+            if (op.kind == kTileDiag) op.wide = {g.wide[0], g.wide[3]};
+            else op.wide = g.wide;
+        }
     };
     auto emit_block = [&](Open& b) {
         if (!b.alive) return;
@@ -672,7 +938,11 @@ std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<Gate
                 fb.gates.push_back(static_cast<uint32_t>(res.size()));
                 res.push_back(resolved(gates[gi]));
             }
-            out.push_back(matrix_op(block_matrix(fb, res), lt, 0, 0, variant));
+            const std::vector<cl> wide = block_matrix_wide(fb, res);
+            std::vector<cd> m;
+            for (const cl& z : wide) m.push_back(narrow(z));
+            out.push_back(matrix_op(m, lt, 0, 0, variant));
+            if (lt.size() == 1 && out.back().kind == kTileDense) out.back().wide = wide;
             return;
         }
         // one matrix per value s of the out-of-tile controls (bit i of s = qubit sel[i]): a
@@ -813,7 +1083,8 @@ std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<Gate
     // one-qubit ops first go into the dense blocks on their qubits (free); the diagonal
     // work left over then merges into tables
     fold_single_qubit_ops(out, max_select);
-    merge_diagonal_runs(out, max_diag, dyn_terms);
+    if (rot) split_rotations(out);
+    else merge_diagonal_runs(out, max_diag, dyn_terms);
     if (store_qubits) {   // qubit each tile bit holds at the end of the pass
         const uint32_t m = cfg.L + static_cast<uint32_t>(item.hbits.size());
         store_qubits->assign(m, 0);
@@ -882,6 +1153,10 @@ uint32_t target_mask(const LocalOp& o) {
     return t;
 }
 
+bool off_diagonal(const LocalOp& o) {
+    return o.kind == kTileDense || o.kind == kTilePauli || o.kind == kTileRot;
+}
+
 // Tile bits an op uses off the diagonal (dense targets) and on it (controls, phase bits,
 // diagonal targets).  Two ops commute when every bit they share is diagonal in both.
 struct Use {
@@ -889,7 +1164,7 @@ struct Use {
 };
 Use op_use(const LocalOp& o) {
     Use u;
-    if (o.kind == kTileDense || o.kind == kTilePauli) u.nd = target_mask(o);
+    if (off_diagonal(o)) u.nd = target_mask(o);
     else if (o.kind == kTileDiag) u.dg = target_mask(o);
     u.dg |= o.lmask;
     return u;
@@ -907,6 +1182,7 @@ struct Lay {
 // register bits.
 bool fits(const LocalOp& o, bool mma, const Lay& ly) {
     if (o.kind == kTilePauli) return (target_mask(o) & ly.W) == 0;   // flips on registers, lanes
+    if (o.kind == kTileRot) return (target_mask(o) & ~ly.S) == 0;
     if (o.kind != kTileDense) return true;
     if (mma) return ly.P != 0 && (target_mask(o) & ~ly.P) == 0 && (o.lmask & ~(ly.S | ly.W)) == 0;
     return (target_mask(o) & ~ly.S) == 0;
@@ -917,7 +1193,7 @@ bool fits(const LocalOp& o, bool mma, const Lay& ly) {
 // ops move there (in order) and `pending` keeps the rest.  mma[i]: op i is a tensor-path op.
 size_t scan(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
             const std::vector<uint8_t>& mma, std::vector<uint32_t>& pending, const Lay& ly,
-            std::vector<uint32_t>* emitted) {
+            std::vector<uint32_t>* emitted, bool rot) {
     uint32_t busy_nd = 0, busy_dg = 0;
     size_t cnt = 0;
     std::vector<uint32_t> rest;
@@ -925,7 +1201,7 @@ size_t scan(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
         const Use& u = use[i];
         const bool blocked = (u.nd & (busy_nd | busy_dg)) != 0 || (u.dg & busy_nd) != 0;
         if (!blocked && fits(ops[i], mma[i] != 0, ly)) {
-            ++cnt;
+            if (!rot || off_diagonal(ops[i])) ++cnt;   // rotation form: diagonals cost no layout
             if (emitted) emitted->push_back(i);
         } else {
             busy_nd |= u.nd;
@@ -943,7 +1219,7 @@ size_t covered(const std::vector<LocalOp>& ops, const std::vector<uint8_t>& mma,
                const std::vector<uint32_t>& pending, uint32_t S) {
     size_t c = 0;
     for (uint32_t i : pending)
-        if ((ops[i].kind == kTileDense || ops[i].kind == kTilePauli) && !mma[i] &&
+        if (off_diagonal(ops[i]) && !mma[i] &&
             (target_mask(ops[i]) & ~S) == 0)
             ++c;
     return c;
@@ -1018,7 +1294,7 @@ uint32_t pick_warp_bits(const std::vector<LocalOp>& ops, const std::vector<uint3
                         uint32_t avail, uint32_t count, uint32_t pair = 0) {
     uint32_t usage[32] = {};
     for (uint32_t i : pending)
-        if (ops[i].kind == kTileDense || ops[i].kind == kTilePauli)
+        if (off_diagonal(ops[i]))
             for (uint32_t b : ops[i].lt) ++usage[b];
     uint32_t W = 0;
     for (uint32_t k = 0; k < count; ++k) {
@@ -1052,7 +1328,7 @@ uint32_t pick_warp_bits(const std::vector<LocalOp>& ops, const std::vector<uint3
 // free of bank conflicts).
 uint32_t choose_set(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
                     const std::vector<uint8_t>& mma, std::vector<uint32_t>& pending,
-                    uint32_t must, uint32_t allowed, uint32_t m, uint32_t lane_pool = 0,
+                    uint32_t must, uint32_t allowed, uint32_t m, bool rot, uint32_t lane_pool = 0,
                     uint32_t P = 0, uint32_t W = 0) {
     uint32_t best = 0;
     size_t best_now = 0, best_later = 0;
@@ -1062,7 +1338,7 @@ uint32_t choose_set(const std::vector<LocalOp>& ops, const std::vector<Use>& use
         if (__builtin_popcount(S) != static_cast<int>(kRegBits) || (S & must) != must ||
             (S & ~allowed) != 0)
             continue;
-        const size_t now = scan(ops, use, mma, pending, Lay{S, W, P}, nullptr);
+        const size_t now = scan(ops, use, mma, pending, Lay{S, W, P}, nullptr, rot);
         const size_t later = covered(ops, mma, pending, S);
         const bool fin = (S & lanes) == 0;
         const bool spread = lane_pool != 0 && residues_spread(lane_pool & ~S);
@@ -1082,6 +1358,14 @@ uint32_t choose_set(const std::vector<LocalOp>& ops, const std::vector<Use>& use
 }  // namespace
 
 namespace {
+
+// A term of a per-tile diagonal, for the entries e with (e & bits) == value: the factor, then
+// {gcmask low 32 bits, gcmask high 32 bits * 4096 + value * 64 + bits} as exact integers.
+void append_term(const cd& f, uint64_t gcmask, uint32_t bits, uint32_t value, std::vector<cd>& mats) {
+    mats.push_back(f);
+    mats.emplace_back(static_cast<double>(gcmask & 0xffffffffu),
+                      static_cast<double>((gcmask >> 32) * 4096u + value * 64u + bits));
+}
 
 // Matrix data of op o in layout (ly, S): dense matrices re-indexed so that matrix bit q is
 // the q-th lowest register target (one block per selector value), diagonals and phase
@@ -1121,20 +1405,16 @@ void append_matrices(const LocalOp& o, const RegLayout& ly, uint32_t S, std::vec
     }
     if (o.kind == kTilePhase || o.kind == kTileDiag) {
         mats.insert(mats.end(), o.m.begin(), o.m.end());
-        // per-tile terms: the factor, then {gcmask low 32 bits, gcmask high 32 bits * 64 +
-        // entry mask} as exact integers
         for (const DynTerm& t : o.dyn) {
-            uint64_t em = 0;
+            uint32_t em = 0;
             for (size_t j = 0; j < o.lt.size(); ++j)
-                if ((t.lbits >> o.lt[j]) & 1) em |= uint64_t{1} << j;
-            mats.push_back(t.f);
-            mats.emplace_back(static_cast<double>(t.gcmask & 0xffffffffu),
-                              static_cast<double>((t.gcmask >> 32) * 64u + em));
+                if ((t.lbits >> o.lt[j]) & 1) em |= 1u << j;
+            append_term(t.f, t.gcmask, em, em, mats);
         }
         return;
     }
     const uint32_t k = static_cast<uint32_t>(o.lt.size());
-    if (k == 1 && !o.variant && o.sel.empty() && is_x(o.m)) return;
+    if (k == 1 && !o.variant && o.sel.empty() && is_x_matrix(o.m)) return;
     int ridx[32];
     for (uint32_t i = 0; i < kRegBits; ++i) ridx[ly.rpos[i]] = static_cast<int>(i);
     uint32_t tm = 0;
@@ -1210,7 +1490,7 @@ RegOp make_record(const LocalOp& o, const RegLayout& ly, uint32_t S, uint32_t m,
         uint32_t tm = 0;
         for (uint32_t b : o.lt) tm |= 1u << ridx[b];
         r.code = static_cast<uint8_t>(tm);
-        r.kind = (k == 1 && !o.variant && o.sel.empty() && is_x(o.m)) ? kRegSwapX : kRegDense;
+        r.kind = (k == 1 && !o.variant && o.sel.empty() && is_x_matrix(o.m)) ? kRegSwapX : kRegDense;
     }
     return r;
 }
@@ -1218,11 +1498,490 @@ RegOp make_record(const LocalOp& o, const RegLayout& ly, uint32_t S, uint32_t m,
 bool same_shape(const LocalOp& a, const LocalOp& b) {
     return a.kind == b.kind && a.lt == b.lt && a.lmask == b.lmask && a.gcmask == b.gcmask &&
            a.sel == b.sel && a.m.size() == b.m.size() && a.variant == b.variant &&
-           a.dyn.size() == b.dyn.size();
+           a.dyn.size() == b.dyn.size() && (a.variant || a.exchange == b.exchange);
+}
+
+// The records of a schedule and the matrices of one state.
+struct Emitted {
+    std::vector<RegOp> rec;
+    std::vector<cd> mats;
+    std::vector<uint32_t> dyn_rec;   // records of per-tile diagonals, and their table entries
+    uint32_t dyn_entries = 0;
+    uint32_t sign_off = 0;           // the sign masks among the matrices
+    double flops = 0.0;
+    // Tile bits stored negated: an X (or the exchange a rotation starts with) costs nothing but
+    // a bit in here, which later records are written for and the tile's store undoes.
+    uint32_t flipped = 0;
+    bool failed = false;             // an operation that cannot be written for a negated bit
+    bool per_state = false;          // some matrix, hence `flipped`, differs per state: the
+                                     // records may depend on neither
+
+    void remap(uint32_t layout, bool local) {
+        close();
+        RegOp r{};
+        r.kind = kRegRemap;
+        r.code = static_cast<uint8_t>(layout);
+        r.k = local ? 1 : 0;
+        rec.push_back(r);
+    }
+    void add(const LocalOp& o, const RegLayout& ly, uint32_t S, uint32_t m, bool mma) {
+        close();
+        push(make_record(o, ly, S, m, static_cast<uint32_t>(mats.size()), mma));
+        append_matrices(o, ly, S, mats, mma);
+        flops += local_op_flops(o, true);
+    }
+    void push(RegOp r) {
+        if (r.kind == kRegDiagDyn || (r.kind == kRegStage && r.nterm)) {
+            (r.kind == kRegStage ? r.dyn_table : r.dyn_off) = static_cast<uint16_t>(dyn_entries);
+            dyn_entries += 1u << r.k;
+            dyn_rec.push_back(static_cast<uint32_t>(rec.size()));
+        }
+        rec.push_back(r);
+    }
+    // Neighbouring rotations on different register bits become one record, with the table that
+    // precedes them.  xy: the rotation's two factors; signs: the outside qubits of the Z on its
+    // bit.
+    void rotate(const LocalOp& o, const RegLayout& ly, const cd& xy, uint64_t signs) {
+        uint32_t r = 0;
+        while (ly.rpos[r] != o.lt[0]) ++r;
+        for (const Rot& x : rots_)
+            if (x.bit == r) {
+                close();
+                break;
+            }
+        rots_.push_back({r, xy, signs});
+        flops += local_op_flops(o, true);
+    }
+    void close() {
+        if (rots_.empty()) return;
+        std::sort(rots_.begin(), rots_.end(), [](const Rot& a, const Rot& b) { return a.bit < b.bit; });
+        const bool after_table = !rec.empty() && rec.back().kind == kRegStage && rec.back().code == 0;
+        if (!after_table) {
+            RegOp r{};
+            r.kind = kRegStage;
+            rec.push_back(r);
+        }
+        RegOp& r = rec.back();
+        r.dyn_off = static_cast<uint16_t>(mats.size());
+        bool any = false;
+        for (const Rot& x : rots_) {
+            r.code = static_cast<uint8_t>(r.code | (1u << x.bit));
+            mats.push_back(x.xy);
+            any |= x.signs != 0;
+        }
+        // where the tile's sign words hold this record's signs; too many of them in one pass:
+        // the masks follow the factors
+        r.tcmask = kRegSignBits;
+        if (any && signs.size() + rots_.size() <= kRegSignBits) {
+            r.tcmask = static_cast<uint16_t>(signs.size());
+            for (const Rot& x : rots_) signs.push_back(x.signs);
+        } else if (any) {
+            r.tcmask = kRegSignBits + 1;
+            for (const Rot& x : rots_) mats.emplace_back(std::bit_cast<double>(x.signs), 0.0);
+        }
+        rots_.clear();
+    }
+    std::vector<uint64_t> signs;     // masks of the rotations' signs, in record order
+
+  private:
+    struct Rot {
+        uint32_t bit;
+        cd xy;
+        uint64_t signs;
+    };
+    std::vector<Rot> rots_;
+};
+
+// Diagonal work of a pass in rotation form that waits for the next operation which needs it:
+// diagonals commute with each other, so each waits until an operation is about to mix one of
+// its tile bits, and then goes out in one table with everything else that fits beside it.
+class DiagonalPool {
+  public:
+    static bool takes(const LocalOp& o) {
+        if (o.kind == kTilePhase)
+            return __builtin_popcount(o.lmask) <= static_cast<int>(kRegMaxDiag);
+        return o.kind == kTileDiag && !o.lmask && !o.gcmask && o.sel.empty() && o.dyn.empty() &&
+               o.lt.size() <= kRegMaxDiag;
+    }
+    void put(const LocalOp& o) { items_.push_back({&o, bits_of(o)}); }
+    bool touches(uint32_t bits) const {
+        for (const Item& it : items_)
+            if (it.bits & bits) return true;
+        return false;
+    }
+    // Emits one table that takes waiting operations on bits of `touch`.
+    void flush(uint32_t touch, Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
+        emit(group(touch), e, ly, S, m);
+    }
+    void flush_all(Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
+        while (!items_.empty()) {
+            uint32_t touch = 0;
+            for (const Item& it : items_) touch |= it.bits;
+            emit(touch ? group(touch) : 0u, e, ly, S, m);
+        }
+    }
+
+  private:
+    struct Item {
+        const LocalOp* op;
+        uint32_t bits;
+    };
+    std::vector<Item> items_;
+
+    static uint32_t bits_of(const LocalOp& o) { return o.kind == kTilePhase ? o.lmask : target_mask(o); }
+    static int width(uint32_t bits) { return __builtin_popcount(bits); }
+
+    // Bits joined to `from` by waiting operations.
+    uint32_t closure(uint32_t from) const {
+        uint32_t c = from;
+        for (bool grew = true; grew;) {
+            grew = false;
+            for (const Item& it : items_)
+                if ((it.bits & c) && (it.bits & ~c)) {
+                    c |= it.bits;
+                    grew = true;
+                }
+        }
+        return c;
+    }
+
+    // Tile bits of the next table: whole components of joined bits while they fit, first those
+    // with a bit of `touch`; if the first is too wide, as much of it as fits.
+    uint32_t group(uint32_t touch) const {
+        const int most = static_cast<int>(kRegMaxDiag);
+        uint32_t u = 0;
+        for (int round = 0; round < 2; ++round)
+            for (const Item& it : items_) {
+                if ((it.bits & u) || (round == 0 && !(it.bits & touch))) continue;
+                const uint32_t c = closure(it.bits);
+                if (!(c & u) && width(u | c) <= most) u |= c;
+            }
+        if (u & touch) return u;
+        u = 0;
+        for (int round = 0; round < 2; ++round)   // what touches, then what is joined to that
+            for (const Item& it : items_)
+                if ((it.bits & (round ? u : touch)) && width(u | it.bits) <= most) u |= it.bits;
+        return u;
+    }
+
+    // One table over the tile bits `u`: the product of every waiting operation within them,
+    // formed in extended precision.  Its entry bits go lanes first (then warp bits, then
+    // register bits), so that the lanes of a warp read neighbouring entries.
+    void emit(uint32_t u, Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
+        RegOp r{};
+        std::vector<uint32_t> bits;
+        for (uint8_t& l : r.loc) l = 31;
+        for (uint32_t i = 0; i < m - kRegBits; ++i)
+            if ((u >> ly.tpos[i]) & 1) {
+                r.loc[bits.size()] = static_cast<uint8_t>(i);
+                bits.push_back(ly.tpos[i]);
+            }
+        uint8_t* const reg_offset[kRegBits] = {&r.nsel, &r.selq[0], &r.selq[1], &r.rcmask};
+        for (uint32_t i = 0; i < kRegBits; ++i)
+            if ((u >> ly.rpos[i]) & 1) {
+                *reg_offset[i] = static_cast<uint8_t>(1u << bits.size());
+                bits.push_back(ly.rpos[i]);
+            }
+        const uint32_t k = static_cast<uint32_t>(bits.size()), size = 1u << k;
+        r.k = static_cast<uint8_t>(k);
+        uint32_t entry_bit[32] = {};
+        for (uint32_t j = 0; j < k; ++j) entry_bit[bits[j]] = 1u << j;
+        auto entry_mask = [&](uint32_t from) {
+            uint32_t x = 0;
+            for (uint32_t b = from; b; b &= b - 1) x |= entry_bit[__builtin_ctz(b)];
+            return x;
+        };
+        const bool dyn_room = e.dyn_rec.size() < kRegMaxDyn && e.dyn_entries + size <= kRegMaxDynEntries;
+        std::vector<const LocalOp*> members, gated, alone;
+        size_t w = 0;
+        for (const Item& it : items_) {
+            if (it.bits & ~u) {
+                items_[w++] = it;
+                continue;
+            }
+            if (it.op->kind != kTilePhase || it.op->gcmask == 0) members.push_back(it.op);
+            else if (dyn_room && gated.size() < kRegMaxDynTerms)
+                gated.push_back(it.op);
+            else alone.push_back(it.op);
+        }
+        items_.resize(w);
+        // a lone phase is cheaper on its own
+        if (members.size() + gated.size() == 1 && !e.per_state && !(u & e.flipped) &&
+            (members.empty() ? gated : members)[0]->kind == kTilePhase) {
+            alone.insert(alone.end(), members.begin(), members.end());
+            alone.insert(alone.end(), gated.begin(), gated.end());
+            members.clear();
+            gated.clear();
+        }
+        if (!members.empty() || !gated.empty()) {
+            const cl one{1, 0};
+            cl bit[kRegMaxDiag][2];
+            for (uint32_t j = 0; j < k; ++j) bit[j][0] = bit[j][1] = one;
+            for (const LocalOp* o : members) {   // one-bit factors first: a product per bit
+                if (o->kind == kTileDiag && o->lt.size() == 1) {
+                    const uint32_t j = static_cast<uint32_t>(__builtin_ctz(entry_bit[o->lt[0]]));
+                    for (int x = 0; x < 2; ++x)
+                        bit[j][x] = wide_mul(bit[j][x], o->wide.empty() ? cl{o->m[x]} : o->wide[x]);
+                } else if (o->kind == kTilePhase && width(o->lmask) == 1) {
+                    cl& f = bit[static_cast<uint32_t>(__builtin_ctz(entry_mask(o->lmask)))][1];
+                    f = wide_mul(f, phase(*o));
+                }
+            }
+            std::vector<cl> table(size, one);
+            for (uint32_t j = 0; j < k; ++j)
+                for (uint32_t x = 0; x < (1u << j); ++x) {
+                    table[x | (1u << j)] = wide_mul(table[x], bit[j][1]);
+                    table[x] = wide_mul(table[x], bit[j][0]);
+                }
+            for (const LocalOp* o : members) {
+                if (o->kind == kTilePhase) {
+                    if (width(o->lmask) == 1) continue;
+                    const uint32_t em = entry_mask(o->lmask);
+                    for (uint32_t x = 0; x < size; ++x)
+                        if ((x & em) == em) table[x] = wide_mul(table[x], phase(*o));
+                } else if (o->lt.size() != 1) {
+                    for (uint32_t x = 0; x < size; ++x) {
+                        uint32_t src = 0;
+                        for (size_t j = 0; j < o->lt.size(); ++j)
+                            if (x & entry_bit[o->lt[j]]) src |= 1u << j;
+                        table[x] = wide_mul(table[x], o->m[src]);
+                    }
+                }
+            }
+            e.close();
+            r.kind = kRegStage;
+            r.pad = 1;
+            r.nterm = static_cast<uint8_t>(gated.size());
+            r.mat_off = static_cast<uint32_t>(e.mats.size());
+            const uint32_t flip = entry_mask(u & e.flipped);
+            for (uint32_t x = 0; x < size; ++x) e.mats.push_back(narrow(table[x ^ flip]));
+            for (const LocalOp* o : gated) {
+                const uint32_t em = entry_mask(o->lmask);
+                append_term(o->m[0], o->gcmask, em, em & ~flip, e.mats);
+            }
+            e.push(r);
+            e.flops += 6.0;
+        }
+        for (const LocalOp* o : alone) {
+            e.failed |= (o->lmask & e.flipped) != 0;
+            e.add(*o, ly, S, m, false);
+        }
+    }
+    static cl phase(const LocalOp& o) { return o.wide.empty() ? cl{o.m[0]} : o.wide[0]; }
+};
+
+// Signs of a pass in rotation form that cost nothing until something cannot take them: a CZ
+// between tile bit b and a qubit outside is a Z on b in the tiles where that qubit is 1, and a
+// CZ between two qubits outside negates whole tiles.
+class PendingSigns {
+  public:
+    explicit PendingSigns(uint32_t m) : m_(m) {}
+    bool take(const LocalOp& o, uint32_t flipped) {
+        if (o.kind != kTilePhase || !o.gcmask || o.m[0] != cd{-1, 0}) return false;
+        if (o.lmask == 0) {
+            if (whole_.size() >= 31u - m_) return false;
+            whole_.push_back(o.gcmask);
+            used_ = true;
+            return true;
+        }
+        if (__builtin_popcount(o.lmask) != 1 || __builtin_popcountll(o.gcmask) != 1) return false;
+        z_[__builtin_ctz(o.lmask)] ^= o.gcmask;
+        if (o.lmask & flipped) odd_ ^= o.gcmask;   // Z X = - X Z
+        used_ = true;
+        return true;
+    }
+    // The outside qubits whose parity puts a Z on an odd number of the tile bits `bits`.
+    uint64_t on(uint32_t bits) const {
+        uint64_t f = 0;
+        for (uint32_t b = bits; b; b &= b - 1) f ^= z_[__builtin_ctz(b)];
+        return f;
+    }
+    bool any(uint32_t bits) const {
+        for (uint32_t b = bits; b; b &= b - 1)
+            if (z_[__builtin_ctz(b)]) return true;
+        return false;
+    }
+    // Applies the signs on the tile bits `bits`; at the end of the pass all that is left.
+    void apply(uint32_t bits, bool last, Emitted& e, const RegLayout& ly) {
+        if (last ? !used_ : !any(bits)) return;
+        e.close();
+        RegOp r{};
+        r.kind = kRegSign;
+        r.mat_off = static_cast<uint32_t>(e.mats.size());
+        auto put = [&](uint64_t f) { e.mats.emplace_back(std::bit_cast<double>(f), 0.0); };
+        auto mask = [&](uint32_t b) {
+            uint64_t f = 0;
+            if ((bits >> b) & 1) std::swap(f, z_[b]);
+            put(f);
+        };
+        for (uint32_t i = 0; i < m_ - kRegBits; ++i) mask(ly.tpos[i]);
+        for (uint32_t i = 0; i < kRegBits; ++i) mask(ly.rpos[i]);
+        put(last ? odd_ : 0);
+        if (last)
+            for (uint64_t f : whole_) put(f);
+        r.nterm = static_cast<uint8_t>(m_ + 1 + (last ? whole_.size() : 0));
+        e.push(r);
+    }
+
+  private:
+    uint32_t m_;
+    uint64_t z_[32] = {};
+    uint64_t odd_ = 0;               // outside qubits whose parity negates the tile
+    std::vector<uint64_t> whole_;    // outside qubits that negate it where they are all 1
+    bool used_ = false;
+};
+
+// Records and matrices of the schedule `seq` for the operations of one state.  In rotation
+// form the operations of one layout go out in the order that leaves diagonals waiting longest:
+// whatever mixes a bit that nothing waits on goes first, and a table is emitted only when
+// every operation that is left needs one.  What waits on the bits that the next layout mixes
+// goes out before the remap, while those bits are thread bits: a thread then loads one entry
+// per register bit of the table that is left.
+void emit_schedule(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
+                   const std::vector<uint8_t>& mma,
+                   const std::vector<std::pair<int, uint32_t>>& seq,
+                   const std::vector<RegLayout>& lays, const std::vector<Lay>& keys, uint32_t m,
+                   const std::vector<uint32_t>& store_q, bool rot, bool flips, Emitted& e) {
+    DiagonalPool pool;
+    std::deque<LocalOp> scales;   // diagonals of mirrored rotations (the pool keeps pointers)
+    uint32_t cur = 0;
+    if (rot) e.mats.emplace_back(0.0, 0.0);   // what the store undoes
+    // bits that controls of records look at are never stored negated
+    uint32_t keep = flips ? 0u : ~0u;
+    for (const LocalOp& o : ops) {
+        e.per_state |= o.variant;
+        if (!DiagonalPool::takes(o) && o.kind != kTilePauli) {
+            keep |= o.lmask;
+            if (o.kind == kTileDiag) keep |= target_mask(o);
+        }
+    }
+    auto exchange = [&](uint32_t bit) {   // the halves of tile bit `bit` trade places
+        if (!((keep >> bit) & 1)) {
+            e.flipped ^= 1u << bit;
+            return;
+        }
+        LocalOp x;
+        x.lt = {bit};
+        x.m = {cd{0, 0}, cd{1, 0}, cd{1, 0}, cd{0, 0}};
+        e.add(x, lays[cur], keys[cur].S, m, false);
+    };
+    PendingSigns signs(m);
+    std::vector<uint32_t> todo, rest;   // of the current layout
+    auto apply = [&](const LocalOp& o) {
+        const RegLayout& ly = lays[cur];
+        const uint32_t t = target_mask(o);
+        const bool x_op = o.kind == kTileDense && !o.variant && !o.lmask && !o.gcmask &&
+                          o.sel.empty() && is_x_matrix(o.m);
+        if (o.kind == kTileRot) {
+            const uint32_t b = o.lt[0];
+            if (o.exchange && ((keep >> b) & 1)) {
+                if (o.variant) e.failed = true;   // records may not differ between states
+                signs.apply(t, false, e, ly);
+            }
+            if (o.exchange) exchange(b);
+            const bool mirrored = (e.flipped & t) != 0;
+            // On a negated bit the rotation is [[1 + x y, y], [x, 1]] = diag(e0, e1) [[1, p],
+            // [q, 1 + p q]]: the same two steps with other factors, and a diagonal that joins
+            // the one waiting behind it (there in every state of a batch).
+            cd xy = o.m[0];
+            cl e0{1, 0}, e1{1, 0};
+            if (mirrored) {
+                const long double x = xy.real(), y = xy.imag(), s = 1.0L + x * y, P = y / s,
+                                  Q = x / (1.0L - P * x);
+                xy = cd{static_cast<double>(P), static_cast<double>(Q)};
+                const long double p = xy.real(), q = xy.imag(), r = 1.0L + p * q;
+                e0 = std::sqrt((s * s + y * y) / (1.0L + p * p));
+                e1 = std::sqrt((x * x + 1.0L) / (q * q + r * r));
+            }
+            e.rotate(o, ly, xy, signs.on(t));
+            if (mirrored || e.per_state) {
+                LocalOp& d = scales.emplace_back();
+                d.kind = kTileDiag;
+                d.lt = o.lt;
+                d.variant = e.per_state;
+                d.wide = {e1, e0};   // of the true bit, the stored one negated
+                d.m = {narrow(e1), narrow(e0)};
+                pool.put(d);
+            }
+        } else if (x_op && !(keep & t)) {
+            e.flipped ^= t;
+        } else if (o.kind == kTilePauli) {
+            LocalOp p = o;   // a Z flips the sign of a string with X or Y on its bit, an X of
+            p.pz_out ^= signs.on(t);   // one with Z or Y
+            if (__builtin_popcount(e.flipped & o.lmask) & 1) p.m[1] = -p.m[1];
+            e.add(p, ly, keys[cur].S, m, false);
+        } else {
+            if (off_diagonal(o)) signs.apply(t, false, e, ly);
+            if (o.kind == kTileDense && (e.flipped & t)) {
+                LocalOp d = o;
+                uint32_t f = 0;
+                for (size_t j = 0; j < o.lt.size(); ++j) f |= ((e.flipped >> o.lt[j]) & 1u) << j;
+                const uint32_t D = 1u << o.lt.size();
+                for (size_t blk = 0; blk < o.m.size(); blk += D * D)
+                    for (uint32_t r = 0; r < D; ++r)
+                        for (uint32_t c = 0; c < D; ++c)
+                            d.m[blk + (r ^ f) * D + (c ^ f)] = o.m[blk + r * D + c];
+                e.add(d, ly, keys[cur].S, m, false);
+                return;
+            }
+            e.add(o, ly, keys[cur].S, m, false);
+        }
+    };
+    auto drain = [&] {
+        while (!todo.empty()) {
+            bool moved = false;
+            uint32_t busy_nd = 0, busy_dg = 0, waits = 0;
+            rest.clear();
+            for (uint32_t i : todo) {
+                const Use& u = use[i];
+                const bool blocked = (u.nd & (busy_nd | busy_dg)) != 0 || (u.dg & busy_nd) != 0;
+                if (!blocked && !off_diagonal(ops[i]) && DiagonalPool::takes(ops[i])) {
+                    if (!signs.take(ops[i], e.flipped)) pool.put(ops[i]);
+                    moved = true;
+                } else if (!blocked && !pool.touches(u.nd)) {
+                    apply(ops[i]);
+                    moved = true;
+                } else {
+                    if (!blocked) waits |= u.nd;
+                    busy_nd |= u.nd;
+                    busy_dg |= u.dg;
+                    rest.push_back(i);
+                }
+            }
+            todo.swap(rest);
+            if (!moved && !todo.empty()) pool.flush(waits, e, lays[cur], keys[cur].S, m);
+        }
+    };
+    for (size_t k = 0; k < seq.size(); ++k) {
+        const auto [i, l] = seq[k];
+        if (i < 0) {
+            drain();
+            uint32_t next = 0;
+            for (size_t j = k + 1; j < seq.size() && seq[j].first >= 0; ++j) next |= use[seq[j].first].nd;
+            while (rot && pool.touches(next)) pool.flush(next, e, lays[cur], keys[cur].S, m);
+            e.remap(l, i == -1);   // warp-local
+        } else if (rot) {
+            todo.push_back(static_cast<uint32_t>(i));
+        } else {
+            e.add(ops[i], lays[l], keys[l].S, m, mma[i] != 0);
+        }
+        cur = l;
+    }
+    drain();
+    pool.flush_all(e, lays[cur], keys[cur].S, m);
+    signs.apply((1u << m) - 1u, true, e, lays[cur]);
+    e.close();
+    if (rot) {
+        uint64_t undo = 0;
+        for (uint32_t b = e.flipped; b; b &= b - 1) undo ^= uint64_t{1} << store_q[__builtin_ctz(b)];
+        e.mats[0] = cd{std::bit_cast<double>(undo), 0.0};
+        e.sign_off = static_cast<uint32_t>(e.mats.size());
+        for (uint64_t f : e.signs) e.mats.emplace_back(std::bit_cast<double>(f), 0.0);
+    }
 }
 
 bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates,
-                        const TileConfig& cfg, uint32_t max_select, RegPass& pass,
+                        const TileConfig& cfg, uint32_t max_select, bool rot, bool flips, RegPass& pass,
                         std::vector<RegOp>& ops_out, std::vector<RegLayout>& layouts_out,
                         std::vector<cd>& mats_out, double* flops_per_amp,
                         const std::vector<std::vector<std::array<cd, 4>>>* state_slots) {
@@ -1231,9 +1990,9 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
         state_slots && !state_slots->empty() ? &(*state_slots)[0] : nullptr;
     std::vector<uint32_t> store_q;
     const std::vector<LocalOp> ops =
-        pass_local_ops(item, gates, cfg, max_select, slots0, kRegMaxDiag, true, &store_q, true);
+        pass_local_ops(item, gates, cfg, max_select, slots0, kRegMaxDiag, true, &store_q, true, rot);
     for (const LocalOp& o : ops)
-        if (o.kind != kTilePhase && o.kind != kTilePauli &&
+        if (o.kind != kTilePhase && o.kind != kTilePauli && o.kind != kTileRot &&
             o.lt.size() > (o.kind == kTileDense ? kRegMaxK : kRegMaxDiag))
             return false;
     std::vector<Use> use;
@@ -1245,7 +2004,7 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     for (size_t i = 0; i < ops.size(); ++i) {
         const LocalOp& o = ops[i];
         const size_t k = o.lt.size();
-        const bool swapx = k == 1 && !o.variant && o.sel.empty() && is_x(o.m);
+        const bool swapx = k == 1 && !o.variant && o.sel.empty() && is_x_matrix(o.m);
         mma[i] = cfg.mma && o.kind == kTileDense && (k == 2 || (k == 1 && !swapx)) &&
                  __builtin_popcount(o.lmask) <= static_cast<int>(kRegBits);
     }
@@ -1298,25 +2057,25 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     };
     // the first layout loads the tile: lanes on tile bits 0..4 keep the loads coalesced
     uint32_t P = next_pair(lanes);
-    uint32_t S = choose_set(ops, use, mma, pending, 0, high, m, 0, P, 0);
+    uint32_t S = choose_set(ops, use, mma, pending, 0, high, m, rot, 0, P, 0);
     uint32_t W = pick_warp_bits(ops, pending, high & ~S, nwarp, P);
     uint32_t cur = layout_index(S, W, P);
     bool sync_tiles = false;
     while (true) {
         std::vector<uint32_t> applied;
-        scan(ops, use, mma, pending, Lay{S, W, P}, &applied);
+        scan(ops, use, mma, pending, Lay{S, W, P}, &applied, rot);
         for (uint32_t i : applied) seq.emplace_back(static_cast<int>(i), cur);
         if (pending.empty()) break;
         const LocalOp& f = ops[pending.front()];
         if (mma[pending.front()]) {   // a tensor-path block: its targets become the lane pair
             P = pair_for(pending.front(), all, all & ~W);
             if ((P & W) == 0) {       // warp-local: the warp bits stay
-                S = choose_set(ops, use, mma, pending, f.lmask & ~W, all & ~W & ~P, m, all & ~W,
+                S = choose_set(ops, use, mma, pending, f.lmask & ~W, all & ~W & ~P, m, rot, all & ~W,
                                P, W);
                 cur = layout_index(S, W, P);
                 seq.emplace_back(-1, cur);
             } else {                  // a target is a warp bit: new warp bits, CTA-wide remap
-                S = choose_set(ops, use, mma, pending, f.lmask, all & ~P, m, 0, P, 0);
+                S = choose_set(ops, use, mma, pending, f.lmask, all & ~P, m, rot, 0, P, 0);
                 W = pick_warp_bits(ops, pending, all & ~S & ~P, nwarp, P);
                 cur = layout_index(S, W, P);
                 seq.emplace_back(-2, cur);
@@ -1326,7 +2085,7 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
         }
         if (f.kind == kTilePauli) {   // its flips on warp bits: new warp bits outside them
             W = pick_warp_bits(ops, pending, all & ~target_mask(f), nwarp);
-            S = choose_set(ops, use, mma, pending, 0, all & ~W, m, all & ~W, 0, W);
+            S = choose_set(ops, use, mma, pending, 0, all & ~W, m, rot, all & ~W, 0, W);
             P = next_pair(all & ~W & ~S);
             cur = layout_index(S, W, P);
             seq.emplace_back(-2, cur);
@@ -1335,12 +2094,12 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
         }
         const uint32_t must = target_mask(f);
         if ((must & W) == 0) {   // warp-local: the warp bits stay
-            S = choose_set(ops, use, mma, pending, must, all & ~W, m, all & ~W, 0, W);
+            S = choose_set(ops, use, mma, pending, must, all & ~W, m, rot, all & ~W, 0, W);
             P = next_pair(all & ~W & ~S);
             cur = layout_index(S, W, P);
             seq.emplace_back(-1, cur);
         } else {                 // a target is a warp bit: new warp bits, CTA-wide remap
-            S = choose_set(ops, use, mma, pending, must, all, m);
+            S = choose_set(ops, use, mma, pending, must, all, m, rot);
             P = next_pair(all & ~S);
             W = pick_warp_bits(ops, pending, all & ~S & ~P, nwarp, P);
             cur = layout_index(S, W, P);
@@ -1371,29 +2130,14 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     }
 
     // records and the first state's matrices
-    std::vector<RegOp> rec;
-    std::vector<cd> mats;
-    std::vector<uint32_t> dyn_rec;
-    uint32_t dyn_entries = 0;
-    for (const auto& [i, l] : seq) {
-        if (i < 0) {
-            RegOp r{};
-            r.kind = kRegRemap;
-            r.code = static_cast<uint8_t>(l);
-            r.k = i == -1 ? 1 : 0;   // 1: warp-local
-            rec.push_back(r);
-            continue;
-        }
-        RegOp r = make_record(ops[i], lays[l], lay_keys[l].S, m, static_cast<uint32_t>(mats.size()),
-                              mma[i] != 0);
-        if (r.kind == kRegDiagDyn) {
-            r.dyn_off = static_cast<uint16_t>(dyn_entries);
-            dyn_entries += 1u << r.k;
-            dyn_rec.push_back(static_cast<uint32_t>(rec.size()));
-        }
-        rec.push_back(r);
-        append_matrices(ops[i], lays[l], lay_keys[l].S, mats, mma[i] != 0);
-    }
+    Emitted first;
+    emit_schedule(ops, use, mma, seq, lays, lay_keys, m, store_q, rot, flips, first);
+    if (first.failed) return false;
+    bool flipped = first.flipped != 0;
+    const std::vector<RegOp>& rec = first.rec;
+    std::vector<cd>& mats = first.mats;
+    const std::vector<uint32_t>& dyn_rec = first.dyn_rec;
+    const uint32_t dyn_entries = first.dyn_entries;
     if (rec.size() > kRegMaxRecords || lays.size() > kRegMaxLayouts || mats.size() > kRegMaxMatrix ||
         dyn_rec.size() > kRegMaxDyn || dyn_entries > kRegMaxDynEntries)
         return false;
@@ -1404,14 +2148,15 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
             std::vector<uint32_t> store_b;
             const std::vector<LocalOp> ob = pass_local_ops(item, gates, cfg, max_select,
                                                            &(*state_slots)[b], kRegMaxDiag, true,
-                                                           &store_b, true);
+                                                           &store_b, true, rot);
             if (ob.size() != ops.size() || store_b != store_q) return false;
             for (size_t i = 0; i < ops.size(); ++i)
                 if (!same_shape(ops[i], ob[i])) return false;
-            const size_t before = mats.size();
-            for (const auto& [i, l] : seq)
-                if (i >= 0) append_matrices(ob[i], lays[l], lay_keys[l].S, mats, mma[i] != 0);
-            if (mats.size() - before != n_mat) return false;
+            Emitted eb;
+            emit_schedule(ob, use, mma, seq, lays, lay_keys, m, store_q, rot, flips, eb);
+            flipped |= eb.flipped != 0;
+            if (eb.failed || eb.mats.size() != n_mat || eb.rec.size() != rec.size()) return false;
+            mats.insert(mats.end(), eb.mats.begin(), eb.mats.end());
         }
     }
     pass = RegPass{};
@@ -1447,10 +2192,16 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     // warps) load: every load of the tile must come before any store.  A CTA-wide remap or
     // the per-tile table barrier, both after the loads, order them; otherwise the kernel
     // adds a barrier after the loads.
-    pass.load_barrier = pass.relabel && !sync_tiles && dyn_rec.empty() ? 1u : 0u;
+    // So does a negated bit.
+    pass.load_barrier = (pass.relabel || flipped) && !sync_tiles && dyn_rec.empty() ? 1u : 0u;
     pass.fma_dense = pass.mma_ops = pass.pauli_ops = 0;
+    pass.last_layout = last_layout;
+    pass.rot = rot ? 1u : 0u;
+    pass.sign_off = first.sign_off;
+    pass.n_signs = static_cast<uint32_t>(first.signs.size());
     for (const RegOp& r : rec) {
-        if (r.kind == kRegDense) pass.fma_dense = 1;
+        if (r.kind == kRegDense || (rot && (r.kind == kRegDiag || r.kind == kRegDiagDyn)))
+            pass.fma_dense = 1;
         if (r.kind == kRegMma) pass.mma_ops = 1;
         if (r.kind == kRegPauli) pass.pauli_ops = 1;
     }
@@ -1458,10 +2209,7 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     ops_out.insert(ops_out.end(), rec.begin(), rec.end());
     layouts_out.insert(layouts_out.end(), lays.begin(), lays.end());
     mats_out.insert(mats_out.end(), mats.begin(), mats.end());
-    if (flops_per_amp) {
-        *flops_per_amp = 0.0;
-        for (const LocalOp& o : ops) *flops_per_amp += local_op_flops(o, true);
-    }
+    if (flops_per_amp) *flops_per_amp = first.flops;
     return true;
 }
 
@@ -1475,10 +2223,14 @@ bool lower_pass_reg(const PlanItem& item, const std::vector<GateDesc>& gates,
     const uint32_t m = cfg.L + static_cast<uint32_t>(item.hbits.size());
     if (m < kRegMinBits || m > kRegMaxBits || item.hbits.size() > kTileMaxHigh) return false;
     // fewer selector qubits when the matrices of a pass outgrow their shared-memory stage
-    for (int sel = static_cast<int>(kRegMaxSelect); sel >= 0; --sel)
-        if (lower_pass_reg_sel(item, gates, cfg, static_cast<uint32_t>(sel), pass, ops_out,
-                               layouts_out, mats_out, flops_per_amp, state_slots))
-            return true;
+    // or, where they still do, or where the states of a batch differ in form (a noise matrix
+    // that has no rotation form in some state), dense operations with merged diagonals; form 2:
+    // rotation form, 1: rotation form without negated bits
+    for (int form = uses_rotation_form(cfg) ? 2 : 0; form >= 0; --form)
+        for (int sel = static_cast<int>(kRegMaxSelect); sel >= 0; --sel)
+            if (lower_pass_reg_sel(item, gates, cfg, static_cast<uint32_t>(sel), form > 0, form == 2,
+                                   pass, ops_out, layouts_out, mats_out, flops_per_amp, state_slots))
+                return true;
     return false;
 }
 

@@ -30,6 +30,20 @@ struct TileConfig {
 bool native_pauli(const GateDesc& g, const TileConfig& cfg);
 TileConfig default_tile_config(uint32_t n);
 
+// Whether register passes take their gates in rotation form (not on the tensor path or in the
+// double-buffered kernel, whose blocks are dense).
+inline bool uses_rotation_form(const TileConfig& cfg) {
+    return cfg.reg && !cfg.mma && !reg_pipe_enabled();
+}
+
+// The same circuit with its entangling gates made diagonal where that costs nothing: an X
+// with controls whose target has a one-qubit (or free two-qubit) gate next to it becomes
+// H Z H, RZZ becomes a controlled phase and two one-qubit diagonals, and runs of one-qubit
+// gates on a qubit multiply into one.  Diagonal gates need no tile slot, so passes hold more
+// gates, and in a pass they merge with the diagonal factors of the one-qubit gates (each of
+// which is diagonal * real rotation * diagonal) into a few tables.
+std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t n);
+
 // A pass (hbits + gates applied in program order) or one gate run on its own.
 struct PlanItem {
     bool is_pass = false;
@@ -37,6 +51,14 @@ struct PlanItem {
     std::vector<uint32_t> hbits;
     std::vector<uint32_t> gates;
 };
+
+// Source gates an item stands for.
+inline uint32_t source_gates(const PlanItem& item, const std::vector<GateDesc>& gates) {
+    if (!item.is_pass) return gates[item.gate].src;
+    uint32_t n = 0;
+    for (uint32_t g : item.gates) n += gates[g].src;
+    return n;
+}
 
 std::vector<PlanItem> plan_tiles(const std::vector<GateDesc>& gates, uint32_t n,
                                  const TileConfig& cfg);
@@ -52,7 +74,7 @@ struct DynTerm {
 
 // One operation of a pass in tile-local bits, before it is encoded for a kernel.
 struct LocalOp {
-    uint8_t kind = kTileDense;      // kTileDense, kTileDiag or kTilePhase
+    uint8_t kind = kTileDense;      // kTileDense, kTileDiag, kTilePhase, kTilePauli, kTileRot
     std::vector<uint32_t> lt;       // targets, matrix local order (none for a phase)
     uint32_t lmask = 0;             // local controls, or the local bits of a phase
     uint64_t gcmask = 0;            // controls / phase bits outside the tile
@@ -61,6 +83,8 @@ struct LocalOp {
     std::vector<cd> m;              // dense: 2^k x 2^k, diagonal: 2^k, phase: the factor;
                                     // with sel, one such block per selector value
     std::vector<DynTerm> dyn;       // diagonal: gated phase terms multiplied into m per tile
+    bool exchange = false;          // kTileRot (m = {(x, y)}): the halves trade places first
+    std::vector<cl> wide;           // m before rounding, where known
     // kTilePauli: lt = the flip (X/Y) bits, lmask = the Z-type (Z/Y) tile bits, pz_out = the
     // Z-type qubits outside the tile, m = {(cos, 0), y} (see kRegPauli)
     uint64_t pz_out = 0;
@@ -73,13 +97,15 @@ struct LocalOp {
 // Runs of commuting diagonal work merge into diagonals of at most max_diag tile bits; with
 // dyn_terms, phases gated by other out-of-tile qubits join them as per-tile terms.  With
 // store_qubits, SWAPs of two tile qubits become relabellings (no operation) and
-// store_qubits[b] receives the qubit whose place tile bit b is stored to.
+// store_qubits[b] receives the qubit whose place tile bit b is stored to.  With rot,
+// uncontrolled one-qubit operations come as diagonal, kTileRot, diagonal, and diagonals are
+// left unmerged (the register lowering merges them as it emits them).
 std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<GateDesc>& gates,
                                     const TileConfig& cfg, uint32_t max_select,
                                     const std::vector<std::array<cd, 4>>* slot_mats = nullptr,
                                     uint32_t max_diag = kTileMaxK, bool dyn_terms = false,
                                     std::vector<uint32_t>* store_qubits = nullptr,
-                                    bool native_rotations = false);
+                                    bool native_rotations = false, bool rot = false);
 
 // Append the tile operations of one pass to ops_out (matrices to arena) and fill `pass`.
 void lower_pass(const PlanItem& item, const std::vector<GateDesc>& gates, const TileConfig& cfg,
