@@ -16,6 +16,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 
 #include "engine.hpp"
 
@@ -138,9 +139,12 @@ namespace {
 // gates, LQCS_ADJ_TILES=0) streams every state per step, and there a batch that stays in L2
 // is faster (32 sets: 4230 against 3210) — max_resident picks that size.
 uint32_t default_resident(uint32_t n, uint64_t batch) {
+    const uint64_t per_set = 2 * (uint64_t{16} << n);
+    // small batches skip the query of free memory (it costs more than a small problem's step)
+    if (per_set * std::min<uint64_t>(batch, 256) <= (uint64_t{16} << 20))
+        return static_cast<uint32_t>(std::min<uint64_t>(batch, 256));
     size_t free_b = 0, total_b = 0;
     cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    const uint64_t per_set = 2 * (uint64_t{16} << n);
     const uint64_t fit = std::max<uint64_t>(1, (free_b / 2) / per_set);
     return static_cast<uint32_t>(std::min<uint64_t>({batch, fit, 256}));
 }
@@ -252,13 +256,26 @@ int env_or(const char* name, int dflt) {
 // terms and the per-set buffers, on a stream of its own.  A call only uploads the new
 // (cos, sin) tables, so the launch sequence of a batch of nb sets never changes: it is
 // captured once as a CUDA graph and replayed (LQCS_GRAPHS=0: launched directly).
+// The two resident state batches of a plan: scratch of one call.  Plans of one shape whose
+// batches are large (above 32 MiB: one call fills the GPU) share a pair, so a new plan of a known
+// shape allocates none and sixteen plans hold little; `mu` is held during a call.
+struct StatePair {
+    int device = 0;
+    uint32_t n = 0, R = 0;
+    std::unique_ptr<lqcs_state> psi, lam;
+    std::mutex mu;
+    size_t bytes() const { return 2 * static_cast<size_t>(R) * (size_t{16} << n); }
+};
+
 struct AdjointPlan {
     uint64_t key = 0;
     uint32_t n = 0, R = 0;
     uint64_t np = 0;
     std::vector<GateStep> steps;
     HamiltonianDev ham;
-    std::unique_ptr<lqcs_state> psi, lam;
+    std::shared_ptr<StatePair> states;
+    lqcs_state *psi = nullptr, *lam = nullptr;   // of states
+    LaunchCtx ctx;
     DeviceBuffer d_cs, d_csi, d_part, d_energy, d_grad;
     // rotation tile passes (empty: one launch per step)
     std::vector<Segment> fwd_segs, bwd_segs;
@@ -266,19 +283,17 @@ struct AdjointPlan {
     cudaStream_t stream = nullptr;
     // (2 nb + with gradients) -> (graph, kernels)
     std::map<uint32_t, std::pair<cudaGraphExec_t, uint64_t>> graphs;
+    std::set<uint32_t> seen;   // keys that have run
 
     AdjointPlan() = default;
     AdjointPlan(const AdjointPlan&) = delete;
     AdjointPlan& operator=(const AdjointPlan&) = delete;
     ~AdjointPlan() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.second.first);
-        psi.reset();
-        lam.reset();
         if (stream) cudaStreamDestroy(stream);
     }
 
     void forward_step(const GateStep& s, uint32_t nb) const {
-        const LaunchCtx& ctx = psi->ctx;
         if (s.param >= 0) {
             launch_pauli_rotation_batched(ctx, psi->d(), n, nb, s.gen.x, s.gen.zy, s.gen.n_y,
                                           d_cs.as<double2>() + static_cast<uint64_t>(s.param) * R);
@@ -288,7 +303,6 @@ struct AdjointPlan {
     }
 
     void backward_step(const GateStep& s, uint32_t nb) const {
-        const LaunchCtx& ctx = psi->ctx;
         if (s.param >= 0) {
             launch_batched_pauli_im_p(ctx, lam->d(), psi->d(), n, nb, s.gen.x, s.gen.zy,
                                       s.gen.n_y, d_part.as<double>(),
@@ -305,7 +319,6 @@ struct AdjointPlan {
     // The launch sequence of one batch of nb sets on this plan's stream; without gradients
     // (energies only) it ends after <psi|H|psi>.
     void enqueue(uint32_t nb, bool grads = true) const {
-        const LaunchCtx& ctx = psi->ctx;
         const uint64_t len = uint64_t{1} << n;
         const RotTileOp* rot_ops = d_rot_ops.as<RotTileOp>();
         launch_set_basis(ctx, psi->d(), n, nb, 0);
@@ -400,6 +413,11 @@ struct AdjointPlan {
         const uint32_t key = 2 * nb + (grads ? 1u : 0u);
         auto it = graphs.find(key);
         bool fresh = false;
+        if (it == graphs.end() && seen.insert(key).second) {
+            // a batch size's first call: capturing and instantiating costs more than it saves
+            enqueue(nb, grads);
+            return;
+        }
         if (it == graphs.end()) {
             // capture once; a failed capture falls back to direct launches (which rethrow any
             // real launch error)
@@ -463,16 +481,20 @@ uint64_t plan_key(const std::vector<GateDesc>& tmpl, const std::vector<int>& par
     return k;
 }
 
-// The most recent plans (resident memory: two state batches each), newest last.
+// The most recent plans, newest last: the last two whatever they hold, and up to sixteen while
+// their resident state batches stay within 1 GiB in all (a loop over a few small problems then
+// plans each once: building a plan takes 1 to 4 ms, a step of a 10-qubit one 0.3).
 std::mutex g_plan_mu;
-std::vector<std::unique_ptr<AdjointPlan>> g_plans;
-constexpr size_t kKeptPlans = 2;
+std::vector<std::shared_ptr<AdjointPlan>> g_plans;
+constexpr size_t kKeptPlans = 2, kMostPlans = 16;
+constexpr size_t kPlanBytes = size_t{1} << 30;
 
 std::unique_ptr<AdjointPlan> build_plan(const std::vector<GateDesc>& tmpl,
                                         const std::vector<int>& param_of, const Hamiltonian& h,
-                                        uint32_t n, uint64_t np, uint32_t R, uint64_t dkey);
+                                        uint32_t n, uint64_t np, uint32_t R, uint64_t dkey,
+                                        std::shared_ptr<StatePair> shared = nullptr);
 
-AdjointPlan& adjoint_plan(const std::vector<GateDesc>& tmpl, const std::vector<int>& param_of,
+std::shared_ptr<AdjointPlan> adjoint_plan(const std::vector<GateDesc>& tmpl, const std::vector<int>& param_of,
                           const Hamiltonian& h, uint32_t n, uint64_t np, uint64_t batch,
                           uint32_t max_resident) {
     const uint32_t R = max_resident ? static_cast<uint32_t>(std::min<uint64_t>(max_resident, batch))
@@ -482,17 +504,35 @@ AdjointPlan& adjoint_plan(const std::vector<GateDesc>& tmpl, const std::vector<i
     cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     const uint64_t dkey = key ^ (static_cast<uint64_t>(dev) << 56);
     std::lock_guard<std::mutex> lk(g_plan_mu);
-    for (auto& p : g_plans)
-        if (p->key == dkey) return *p;
-    auto plan = build_plan(tmpl, param_of, h, n, np, R, dkey);
-    if (g_plans.size() >= kKeptPlans) g_plans.erase(g_plans.begin());
-    g_plans.push_back(std::move(plan));
-    return *g_plans.back();
+    for (auto it = g_plans.begin(); it != g_plans.end(); ++it)
+        if ((*it)->key == dkey) {
+            std::rotate(it, it + 1, g_plans.end());
+            return g_plans.back();
+        }
+    std::shared_ptr<StatePair> shared;
+    const size_t need = 2 * static_cast<size_t>(R) * (size_t{16} << n);
+    if (need > (size_t{32} << 20))
+        for (const auto& p : g_plans)
+            if (p->states->device == dev && p->n == n && p->R == R) shared = p->states;
+    auto held = [&] {
+        size_t b = shared ? 0 : need;
+        for (size_t i = 0; i < g_plans.size(); ++i) {
+            bool first = true;
+            for (size_t j = 0; j < i; ++j) first &= g_plans[j]->states != g_plans[i]->states;
+            if (first) b += g_plans[i]->states->bytes();
+        }
+        return b;
+    };
+    while (g_plans.size() >= kMostPlans || (g_plans.size() >= kKeptPlans && held() > kPlanBytes))
+        g_plans.erase(g_plans.begin());
+    g_plans.push_back(build_plan(tmpl, param_of, h, n, np, R, dkey, shared));
+    return g_plans.back();
 }
 
 std::unique_ptr<AdjointPlan> build_plan(const std::vector<GateDesc>& tmpl,
                                         const std::vector<int>& param_of, const Hamiltonian& h,
-                                        uint32_t n, uint64_t np, uint32_t R, uint64_t dkey) {
+                                        uint32_t n, uint64_t np, uint32_t R, uint64_t dkey,
+                                        std::shared_ptr<StatePair> shared) {
     auto plan = std::make_unique<AdjointPlan>();
     plan->key = dkey;
     plan->n = n;
@@ -515,8 +555,19 @@ std::unique_ptr<AdjointPlan> build_plan(const std::vector<GateDesc>& tmpl,
         }
         plan->steps.push_back(std::move(s));
     }
-    plan->psi = new_state(n, R, plan->stream);
-    plan->lam = new_state(n, R, plan->stream);
+    plan->ctx = make_ctx(plan->stream);
+    plan->states = shared ? shared : std::make_shared<StatePair>();
+    if (!shared) {
+        StatePair& sp = *plan->states;
+        cuda_check(cudaGetDevice(&sp.device), "cudaGetDevice");
+        sp.n = n;
+        sp.R = R;
+        sp.psi = new_state(n, R, nullptr);
+        sp.lam = new_state(n, R, nullptr);
+        sp.psi->sync();   // the plan works on a stream of its own
+    }
+    plan->psi = plan->states->psi.get();
+    plan->lam = plan->states->lam.get();
     plan->ham.upload(h, n);
     plan->plan_tiles();
     plan->d_cs.ensure(sizeof(double2) * std::max<uint64_t>(1, np) * R);
@@ -589,7 +640,9 @@ void adjoint_batched(const lqcs_parametric_circuit* pc, const Hamiltonian& h,
         return;
     }
 
-    AdjointPlan& plan = adjoint_plan(tmpl, param_of, h, n, np, batch, max_resident);
+    const std::shared_ptr<AdjointPlan> held = adjoint_plan(tmpl, param_of, h, n, np, batch, max_resident);
+    AdjointPlan& plan = *held;   // alive although another call may drop it from the list
+    std::lock_guard<std::mutex> busy(plan.states->mu);
     const uint32_t R = plan.R;
     std::vector<double2> cs(np * R), csi(np * R);
     std::vector<double> h_energy(R), h_grad(np * R);

@@ -25,21 +25,169 @@ void cuda_check(cudaError_t e, const char* what) {
     throw Error(LQCS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+namespace {
+
+constexpr size_t kBlockMax = size_t{32} << 20, kIdleMax = size_t{256} << 20;
+// Blocks of up to 1 MiB are cut from slabs of 8 MiB: a plan or a program needs a dozen of them.
+constexpr size_t kSlabBlockMax = size_t{1} << 20, kSlab = size_t{8} << 20;
+
+struct BlockPool {
+    struct Slab {
+        char* base;
+        size_t used;   // bytes cut so far
+        size_t live;   // blocks in use
+    };
+    std::mutex mu;
+    std::map<std::pair<int, size_t>, std::vector<void*>> idle;
+    std::map<int, size_t> idle_bytes;
+    std::map<int, std::vector<Slab>> slabs;
+
+    Slab* slab_of(int device, void* p) {
+        for (Slab& s : slabs[device])
+            if (p >= s.base && p < s.base + kSlab) return &s;
+        return nullptr;
+    }
+    // Idle blocks and slabs without a block in use, taken out of the pool (to be freed).
+    std::vector<std::pair<int, void*>> take_idle() {
+        std::vector<std::pair<int, void*>> drop;
+        for (auto& [key, ptrs] : idle) {
+            std::vector<void*> keep;
+            for (void* p : ptrs) {
+                const Slab* s = key.second <= kSlabBlockMax ? slab_of(key.first, p) : nullptr;
+                if (s && s->live > 0) {
+                    keep.push_back(p);
+                    continue;
+                }
+                idle_bytes[key.first] -= key.second;
+                if (!s) drop.emplace_back(key.first, p);
+            }
+            ptrs.swap(keep);
+        }
+        for (auto& [dev, list] : slabs) {
+            std::vector<Slab> keep;
+            for (const Slab& s : list) {
+                if (s.live > 0) keep.push_back(s);
+                else drop.emplace_back(dev, s.base);
+            }
+            list.swap(keep);
+        }
+        return drop;
+    }
+};
+BlockPool& blocks() {   // never destroyed: buffers may be freed during process exit
+    static auto* p = new BlockPool;
+    return *p;
+}
+
+void free_all(const std::vector<std::pair<int, void*>>& drop) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    for (const auto& [dev, p] : drop) {
+        cudaSetDevice(dev);
+        cudaFree(p);
+    }
+    if (!drop.empty()) cudaSetDevice(cur);
+}
+
+// Capacity of a block for b bytes: the next of 4, 5, 6, 7 times a power of two, 512 at least.
+size_t block_size(size_t b) {
+    size_t step = 128;
+    while (step * 8 < b) step <<= 1;
+    return std::max<size_t>(512, (b + step - 1) / step * step);
+}
+
+}  // namespace
+
+void clear_buffer_pool() {
+    std::vector<std::pair<int, void*>> drop;
+    {
+        std::lock_guard<std::mutex> lk(blocks().mu);
+        drop = blocks().take_idle();
+    }
+    free_all(drop);
+}
+
 void DeviceBuffer::release() {
-    if (ptr) cudaFree(ptr);
+    if (!ptr) return;
+    void* p = ptr;
+    const size_t b = bytes;
     ptr = nullptr;
     bytes = 0;
+    if (b > kBlockMax) {
+        cudaFree(p);
+        return;
+    }
+    int cur = 0;
+    const bool known = cudaGetDevice(&cur) == cudaSuccess;
+    if (known && cur != device) cudaSetDevice(device);
+    const bool done = known && cudaDeviceSynchronize() == cudaSuccess;
+    if (known && cur != device) cudaSetDevice(cur);
+    std::vector<std::pair<int, void*>> drop;
+    {
+        std::lock_guard<std::mutex> lk(blocks().mu);
+        BlockPool::Slab* s = b <= kSlabBlockMax ? blocks().slab_of(device, p) : nullptr;
+        if (!done) {
+            // the device did not come to rest (a failed context, process exit): a block of its
+            // own goes back to the driver, one cut from a slab is never handed out again
+            if (!s) drop.emplace_back(device, p);
+        } else {
+            if (s) --s->live;
+            size_t& total = blocks().idle_bytes[device];
+            blocks().idle[{device, b}].push_back(p);
+            total += b;
+            if (total > kIdleMax) drop = blocks().take_idle();
+        }
+    }
+    free_all(drop);
 }
 
 void DeviceBuffer::ensure(size_t b) {
     if (b <= bytes) return;
-    if (ptr) {
-        cuda_check(cudaFree(ptr), "cudaFree");
-        ptr = nullptr;
-        bytes = 0;
+    release();
+    cuda_check(cudaGetDevice(&device), "cudaGetDevice");
+    const size_t want = b <= kBlockMax ? block_size(b) : b;
+    const bool slab = want <= kSlabBlockMax;
+    // an idle block, or one cut from a slab
+    auto take = [&](bool cut) -> void* {
+        BlockPool& pool = blocks();
+        const auto it = pool.idle.find({device, want});
+        if (it != pool.idle.end() && !it->second.empty()) {
+            void* p = it->second.back();
+            it->second.pop_back();
+            pool.idle_bytes[device] -= want;
+            if (BlockPool::Slab* s = slab ? pool.slab_of(device, p) : nullptr) ++s->live;
+            return p;
+        }
+        if (!cut) return nullptr;
+        for (BlockPool::Slab& s : pool.slabs[device])
+            if (s.used + want <= kSlab) {
+                void* p = s.base + s.used;
+                s.used += want;
+                ++s.live;
+                return p;
+            }
+        return nullptr;
+    };
+    if (want <= kBlockMax) {
+        std::lock_guard<std::mutex> lk(blocks().mu);
+        ptr = take(slab);
     }
-    cuda_check(cudaMalloc(&ptr, b), "cudaMalloc");
-    bytes = b;
+    if (!ptr) {
+        void* fresh = nullptr;
+        cudaError_t e = cudaMalloc(&fresh, slab ? kSlab : want);
+        if (e == cudaErrorMemoryAllocation) {   // once more without the idle blocks
+            cudaGetLastError();
+            clear_buffer_pool();
+            e = cudaMalloc(&fresh, slab ? kSlab : want);
+        }
+        cuda_check(e, "cudaMalloc");
+        if (slab) {
+            std::lock_guard<std::mutex> lk(blocks().mu);
+            blocks().slabs[device].push_back({static_cast<char*>(fresh), want, 1});
+        }
+        ptr = fresh;
+    }
+    bytes = want;
 }
 
 int device_sm_count() {
@@ -634,7 +782,7 @@ uint32_t max_qubits_on_device(uint32_t batch) {
     return q;
 }
 
-// Freed amplitude buffers of at most 1 GiB (a 26-qubit state), kept for the next state of the
+// Freed amplitude buffers of 32 MiB to 1 GiB (a 26-qubit state), kept for the next state of the
 // same size on the same device: short runs (sampling loops, small circuits, trajectory
 // batches of small states) skip cudaMalloc and cudaFree, which synchronise the device.  At
 // most four buffers are kept; lqcs_release_caches frees them.
@@ -687,7 +835,8 @@ void clear_state_pool() {
 }
 
 void pool_return(lqcs_state& st) {
-    if (!st.amps.ptr || st.amps.bytes > kPoolMaxBytes) return;
+    // (smaller ones are the block pool's)
+    if (!st.amps.ptr || st.amps.bytes <= kBlockMax || st.amps.bytes > kPoolMaxBytes) return;
     // the buffer is reused only after this state's work on it has finished
     if (cudaStreamSynchronize(st.stream) != cudaSuccess) return;
     void* evict = nullptr;
@@ -715,12 +864,19 @@ void pool_return(lqcs_state& st) {
 std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t stream) {
     if (n == 0) invalid("Statevector: num_qubits must be >= 1");
     if (batch == 0) invalid("state batch must be >= 1");
-    const uint32_t cap = max_qubits_on_device(batch);
-    if (n > cap || n > 40) {
+    auto too_large = [&](uint32_t cap) {
         const double gib = 16.0 * std::ldexp(1.0, static_cast<int>(n) - 30) * batch;
         invalid("Statevector: " + std::to_string(n) + " qubits would need " +
                 std::to_string(gib) + " GiB (max " + std::to_string(cap) +
                 " qubits on this device)");
+    };
+    // small states skip the query of free memory (it costs more than their kernels): the
+    // allocation itself tells
+    const bool small = n <= 40 && (static_cast<double>(batch) * std::ldexp(16.0, static_cast<int>(n))) <=
+                                      static_cast<double>(kBlockMax);
+    if (!small) {
+        const uint32_t cap = max_qubits_on_device(batch);
+        if (n > cap || n > 40) too_large(cap);
     }
     auto st = std::make_unique<lqcs_state>();
     cuda_check(cudaGetDevice(&st->device), "cudaGetDevice");
@@ -732,8 +888,14 @@ std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t s
     if (void* p = pool_take(st->device, bytes)) {
         st->amps.ptr = p;
         st->amps.bytes = bytes;
+        st->amps.device = st->device;
     } else {
-        st->amps.ensure(bytes);
+        try {
+            st->amps.ensure(bytes);
+        } catch (const Error& e) {
+            if (!small || e.code != LQCS_ERR_OUT_OF_MEMORY) throw;
+            too_large(max_qubits_on_device(batch));
+        }
     }
     launch_set_basis(st->ctx, st->d(), n, batch, 0);
     return st;
@@ -794,6 +956,8 @@ std::string program_key(const std::vector<GateDesc>& gates, uint32_t n, const Fu
     return k;
 }
 
+}  // namespace
+
 std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
                                               const FusionConfig& fc, cudaStream_t stream) {
     if (fc.fuse && (fc.mode == kFuseLearned || fc.mode == kFuseAutotune))
@@ -817,8 +981,6 @@ std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates
     if (progs().size() > kProgramCache) progs().pop_front();
     return prog;
 }
-
-}  // namespace
 
 void clear_program_cache() {
     std::lock_guard<std::mutex> lk(prog_mu());

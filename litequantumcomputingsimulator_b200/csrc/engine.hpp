@@ -16,19 +16,28 @@ namespace lqcs_b200 {
 
 void cuda_check(cudaError_t e, const char* what);
 
-// Owning device allocation.
+// Owning device allocation.  Blocks of up to 32 MiB come from and go back to a pool that all
+// buffers of a device share (at most 256 MiB lie idle in it; lqcs_release_caches and a failed
+// allocation empty it): cudaMalloc and cudaFree cost 0.1 to 10 ms a call on a shared host, more
+// than the kernels of a 20-qubit run.  Like cudaFree, release() first waits for the device, so
+// a block is idle when it is handed out again, whatever streams used it.
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
+    int device = 0;
     DeviceBuffer() = default;
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-    DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes) { o.ptr = nullptr; o.bytes = 0; }
+    DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes), device(o.device) {
+        o.ptr = nullptr;
+        o.bytes = 0;
+    }
     DeviceBuffer& operator=(DeviceBuffer&& o) noexcept {
         if (this != &o) {
             release();
             ptr = o.ptr;
             bytes = o.bytes;
+            device = o.device;
             o.ptr = nullptr;
             o.bytes = 0;
         }
@@ -103,6 +112,11 @@ uint32_t default_fusion_width();
 void clear_program_cache();
 // Free the amplitude buffers kept for new states of the same size.
 void clear_state_pool();
+// Free the idle blocks of the buffer pool.
+void clear_buffer_pool();
+// The compiled program of a gate list: one of the last few circuits' or a new one.
+std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
+                                              const FusionConfig& fc, cudaStream_t stream);
 // Called by ~lqcs_state: keeps a small amplitude buffer for the next state of its size.
 void pool_return(lqcs_state& st);
 

@@ -420,11 +420,10 @@ bool run_shared_prefix(uint32_t n, const std::vector<Item>& items,
 
     auto st = new_state(n, 1, nullptr);
     const LaunchCtx ctx = st->ctx;
-    launch_set_basis(ctx, st->d(), n, 1, 0);
-    Program prog;
+    std::shared_ptr<const Program> prog;
     if (!prefix.empty()) {
-        prog = compile(prefix, n, fc, nullptr);
-        prog.launch(ctx, st->d(), n, 1);
+        prog = cached_program(prefix, n, fc, nullptr);
+        prog->launch(ctx, st->d(), n, 1);
     }
     const uint64_t entries = uint64_t{1} << m;
     DeviceBuffer partial, table;
