@@ -16,8 +16,10 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <numbers>
 #include <set>
 
+#include "adj_pass.cuh"
 #include "engine.hpp"
 
 namespace lqcs_b200 {
@@ -97,19 +99,20 @@ DevOp invert(const DevOp& op) {
 // Terms as c_t i^{n_y} with their masks, grouped by the bits of x above the kernel's tile
 // (stable within a group, groups by first appearance).
 void HamiltonianDev::upload(const Hamiltonian& h, uint32_t n) {
-    static const cd ipow[4] = {{1, 0}, {0, 1}, {-1, 0}, {0, -1}};
     const uint32_t ml = ham_tile_bits(n);
     std::vector<uint64_t> keys;
     std::vector<std::vector<PauliTermDev>> by_key;
     for (size_t t = 0; t < h.terms.size(); ++t) {
-        const cd c = h.coeffs[t] * ipow[h.terms[t].n_y % 4];
+        const PauliMasks& p = h.terms[t];
+        const uint32_t power = (p.n_y + 2u * static_cast<uint32_t>(__builtin_popcountll(p.x & p.zy) & 1)) & 3u;
+        const double w = power & 2u ? -h.coeffs[t] : h.coeffs[t];
         const uint64_t key = h.terms[t].x >> ml;
         size_t k = std::find(keys.begin(), keys.end(), key) - keys.begin();
         if (k == keys.size()) {
             keys.push_back(key);
             by_key.emplace_back();
         }
-        by_key[k].push_back({h.terms[t].x, h.terms[t].zy, make_double2(c.real(), c.imag())});
+        by_key[k].push_back({p.zy, w, static_cast<uint32_t>(p.x & ((uint64_t{1} << ml) - 1)), power & 1u});
     }
     std::vector<PauliTermDev> flat;
     std::vector<uint32_t> grp{static_cast<uint32_t>(keys.size())};
@@ -153,10 +156,78 @@ uint32_t default_resident(uint32_t n, uint64_t batch) {
 
 namespace {
 
-// One launch of the forward or backward sweep: a rotation tile pass (step < 0; its ops at
-// op_off in d_rot_ops) or one step launched on its own.
+// A Pauli operator i^k X^x Z^z (Z acts first).
+struct PauliOp {
+    uint64_t x = 0, z = 0;
+    uint32_t k = 0;
+    friend PauliOp operator*(const PauliOp& a, const PauliOp& b) {
+        return {a.x ^ b.x, a.z ^ b.z,
+                (a.k + b.k + 2u * static_cast<uint32_t>(__builtin_popcountll(a.z & b.x) & 1)) & 3u};
+    }
+};
+
+// P -> C^dagger P C for the product C of the Clifford gates so far, as the images of every X_q
+// and Z_q.
+class CliffordFrame {
+  public:
+    explicit CliffordFrame(uint32_t n) : x_(n), z_(n) {
+        for (uint32_t q = 0; q < n; ++q) {
+            x_[q].x = uint64_t{1} << q;
+            z_[q].z = uint64_t{1} << q;
+        }
+    }
+    PauliMasks operator()(const PauliMasks& p) const {
+        PauliOp r{0, 0, p.n_y & 3u};
+        for (uint64_t b = p.x; b; b &= b - 1) r = r * x_[__builtin_ctzll(b)];
+        for (uint64_t b = p.zy; b; b &= b - 1) r = r * z_[__builtin_ctzll(b)];
+        PauliMasks m;
+        m.x = r.x;
+        m.zy = r.z;
+        m.n_y = r.k;
+        return m;
+    }
+    // C <- g C, whose images are those of g^dagger X_q g and g^dagger Z_q g; false if g is not one
+    // of the Clifford gates known here.
+    bool apply(const GateDesc& g) {
+        const uint32_t q = g.targets()[0];
+        PauliOp &X = x_[q], &Z = z_[q];
+        const PauliOp minus{0, 0, 2}, i{0, 0, 1}, minus_i{0, 0, 3};
+        if (g.n_controls == 0) {
+            switch (g.type) {
+                case LQCS_GATE_I: return true;
+                case LQCS_GATE_X: Z = minus * Z; return true;
+                case LQCS_GATE_Y: X = minus * X; Z = minus * Z; return true;
+                case LQCS_GATE_Z: X = minus * X; return true;
+                case LQCS_GATE_H: std::swap(X, Z); return true;
+                case LQCS_GATE_S: X = minus_i * X * Z; return true;    // -Y
+                case LQCS_GATE_SDG: X = i * X * Z; return true;        // Y
+                case LQCS_GATE_SX: Z = i * X * Z; return true;         // Y
+                case LQCS_GATE_SWAP:
+                    std::swap(x_[q], x_[g.targets()[1]]);
+                    std::swap(z_[q], z_[g.targets()[1]]);
+                    return true;
+                default: return false;
+            }
+        }
+        if (g.n_controls != 1) return false;
+        PauliOp &Xc = x_[g.controls()[0]], &Zc = z_[g.controls()[0]];
+        switch (g.type) {
+            case LQCS_GATE_X: Xc = Xc * X; Z = Zc * Z; return true;
+            case LQCS_GATE_Z: Xc = Xc * Z; X = Zc * X; return true;
+            case LQCS_GATE_Y: Xc = Xc * (i * X * Z); X = Zc * X; Z = Zc * Z; return true;
+            default: return false;
+        }
+    }
+
+  private:
+    std::vector<PauliOp> x_, z_;
+};
+
+// One launch of the forward or backward sweep: a register pass of rotations (adj >= 0), a
+// rotation tile pass (its ops at op_off in d_rot_ops) or one step launched on its own.
 struct Segment {
     int step = -1;
+    int adj = -1;
     RotTilePass pass{};
     uint32_t op_off = 0;
 };
@@ -271,7 +342,10 @@ struct AdjointPlan {
     uint64_t key = 0;
     uint32_t n = 0, R = 0;
     uint64_t np = 0;
+    uint64_t np_all = 0;               // np and the fixed rotations' rows of the angle tables
+    std::vector<double> fixed;         // their angles
     std::vector<GateStep> steps;
+    std::vector<AdjPass> fwd_passes, bwd_passes;
     HamiltonianDev ham;
     std::shared_ptr<StatePair> states;
     lqcs_state *psi = nullptr, *lam = nullptr;   // of states
@@ -306,7 +380,7 @@ struct AdjointPlan {
         if (s.param >= 0) {
             launch_batched_pauli_im_p(ctx, lam->d(), psi->d(), n, nb, s.gen.x, s.gen.zy,
                                       s.gen.n_y, d_part.as<double>(),
-                                      d_grad.as<double>() + s.param, np);
+                                      d_grad.as<double>() + s.param, np_all);
             const double2* inv = d_csi.as<double2>() + static_cast<uint64_t>(s.param) * R;
             launch_pauli_rotation_batched(ctx, psi->d(), n, nb, s.gen.x, s.gen.zy, s.gen.n_y, inv);
             launch_pauli_rotation_batched(ctx, lam->d(), n, nb, s.gen.x, s.gen.zy, s.gen.n_y, inv);
@@ -327,6 +401,8 @@ struct AdjointPlan {
         } else {
             for (const Segment& sg : fwd_segs) {
                 if (sg.step >= 0) forward_step(steps[sg.step], nb);
+                else if (sg.adj >= 0) launch_adj_fwd(ctx, psi->d(), n, nb, fwd_passes[sg.adj],
+                                                     d_cs.as<double2>(), R);
                 else launch_rot_tile_fwd(ctx, psi->d(), n, nb, sg.pass, rot_ops + sg.op_off,
                                          d_cs.as<double2>(), R);
             }
@@ -345,16 +421,20 @@ struct AdjointPlan {
         } else {
             for (const Segment& sg : bwd_segs) {
                 if (sg.step >= 0) backward_step(steps[sg.step], nb);
+                else if (sg.adj >= 0) launch_adj_bwd(ctx, psi->d(), lam->d(), n, nb, bwd_passes[sg.adj],
+                                                     d_cs.as<double2>(), R, d_rot_part.as<double>(),
+                                                     d_grad.as<double>(), np_all);
                 else launch_rot_tile_bwd(ctx, psi->d(), lam->d(), n, nb, sg.pass, rot_ops + sg.op_off,
                                          d_cs.as<double2>(), R, d_rot_part.as<double>(),
-                                         d_grad.as<double>(), np);
+                                         d_grad.as<double>(), np_all);
             }
         }
     }
 
-    // Rotation tile passes for both sweeps: forward tiles of 2^min(n, 12) amplitudes (one
-    // state in shared memory), backward 2^min(n, 11) (psi and lambda); qubits 0..2 stay in
-    // every tile so tile rows are 128-byte lines.  LQCS_ADJ_TILES=0 keeps one launch per step.
+    // Passes of rotations for both sweeps: register passes (adj_pass.cuh) from 9 qubits, forward
+    // tiles of 2^min(n, 12) amplitudes (16 per thread), backward 2^min(n, 11) (8 of psi and 8 of
+    // lambda); below, where a tile has fewer amplitudes than a warp's registers, rotation tile
+    // passes in shared memory.  LQCS_ADJ_TILES=0 keeps one launch per step.
     void plan_tiles() {
         if (env_or("LQCS_ADJ_TILES", 1) == 0) return;
         const uint32_t mf = std::min<uint32_t>(n, static_cast<uint32_t>(env_or("LQCS_ADJ_TILE_F", 12)));
@@ -365,6 +445,22 @@ struct AdjointPlan {
         std::vector<const GateStep*> run;
         std::vector<size_t> idx;
         auto flush = [&](std::vector<Segment>& segs, uint32_t m) {
+            if (n >= kAdjMinBits && m >= kAdjMinBits) {
+                const bool back = &segs == &bwd_segs;
+                std::vector<AdjRotation> rots;
+                for (const GateStep* s : run)
+                    rots.push_back({s->gen.x, s->gen.zy, s->gen.n_y, static_cast<uint32_t>(s->param)});
+                std::vector<AdjPass>& passes = back ? bwd_passes : fwd_passes;
+                for (AdjPass& p : plan_adjoint_passes(rots, n, m, back ? kAdjBwdRegs : kAdjFwdRegs)) {
+                    Segment sg;
+                    sg.adj = static_cast<int>(passes.size());
+                    segs.push_back(sg);
+                    passes.push_back(p);
+                }
+                run.clear();
+                idx.clear();
+                return;
+            }
             plan_rotation_passes(run, idx, n, m, L, segs, ops);
             run.clear();
             idx.clear();
@@ -395,7 +491,8 @@ struct AdjointPlan {
         flush(bwd_segs, mb);
         uint32_t max_ops = 1;
         for (const Segment& sg : bwd_segs)
-            if (sg.step < 0) max_ops = std::max(max_ops, sg.pass.n_ops);
+            if (sg.step < 0)
+                max_ops = std::max(max_ops, sg.adj >= 0 ? bwd_passes[sg.adj].n_rots : sg.pass.n_ops);
         d_rot_ops.ensure(sizeof(RotTileOp) * std::max<size_t>(1, ops.size()));
         if (!ops.empty())
             cuda_check(cudaMemcpy(d_rot_ops.ptr, ops.data(), sizeof(RotTileOp) * ops.size(),
@@ -539,8 +636,62 @@ std::unique_ptr<AdjointPlan> build_plan(const std::vector<GateDesc>& tmpl,
     plan->R = R;
     plan->np = np;
     cuda_check(cudaStreamCreateWithFlags(&plan->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    // Without fixed gates in the way every rotation can join a pass: Clifford gates move to the
+    // end of the circuit, where they only change the Hamiltonian's strings (E = <0|U^dagger
+    // C^dagger H C U|0>), each turning the Pauli strings of the rotations it passes into other
+    // strings; a fixed rotation (T, P, RZ, ...; up to a phase) is a rotation whose angle is a
+    // constant.  36 CX between the rotations of a 10-qubit ansatz were 108 launches of 0.34 ms.
+    const Hamiltonian* hh = &h;
+    Hamiltonian moved;
+    if (env_or("LQCS_ADJ_TILES", 1) != 0) {
+        CliffordFrame frame(n);
+        std::vector<GateStep> steps;
+        std::vector<double> fixed;
+        bool ok = true;
+        for (size_t i = 0; ok && i < tmpl.size(); ++i) {
+            const GateDesc& g = tmpl[i];
+            if (g.type == LQCS_GATE_RESET) invalid("run_statevector: Reset is non-deterministic; use run() instead");
+            if (!g.is_unitary()) continue;
+            GateStep s;
+            if (param_of[i] >= 0) {
+                s.param = param_of[i];
+                s.gen = frame(generator(g));
+            } else if (g.n_controls == 0 && !g.slot &&
+                       (g.type == LQCS_GATE_T || g.type == LQCS_GATE_TDG || g.type == LQCS_GATE_P ||
+                        g.type == LQCS_GATE_RX || g.type == LQCS_GATE_RY || g.type == LQCS_GATE_RZ ||
+                        g.type == LQCS_GATE_PAULI_ROTATION)) {
+                GateDesc r = g;
+                double angle = std::numbers::pi / 4;
+                if (g.type == LQCS_GATE_TDG) angle = -angle;
+                else if (g.type != LQCS_GATE_T) angle = g.params.at(0);
+                if (g.type == LQCS_GATE_T || g.type == LQCS_GATE_TDG || g.type == LQCS_GATE_P)
+                    r.type = LQCS_GATE_RZ;
+                s.param = static_cast<int>(np + fixed.size());
+                s.gen = frame(generator(r));
+                fixed.push_back(angle);
+            } else {
+                ok = frame.apply(g);
+                continue;
+            }
+            if (s.gen.x || s.gen.zy) steps.push_back(std::move(s));
+        }
+        // (a parameter whose string is the identity has gradient 0 and keeps its launch)
+        for (size_t i = 0; ok && i < tmpl.size(); ++i)
+            if (param_of[i] >= 0) {
+                const PauliMasks m = generator(tmpl[i]);
+                ok = m.x || m.zy;
+            }
+        if (ok) {
+            plan->steps = std::move(steps);
+            plan->fixed = std::move(fixed);
+            moved = h;
+            for (PauliMasks& t : moved.terms) t = frame(t);
+            hh = &moved;
+        }
+    }
+    plan->np_all = np + plan->fixed.size();
     // the fixed gates (and their inverses); barrier / measure are skipped
-    for (size_t i = 0; i < tmpl.size(); ++i) {
+    for (size_t i = 0; hh == &h && i < tmpl.size(); ++i) {
         const GateDesc& g = tmpl[i];
         if (g.type == LQCS_GATE_RESET) invalid("run_statevector: Reset is non-deterministic; use run() instead");
         if (!g.is_unitary()) continue;
@@ -568,13 +719,13 @@ std::unique_ptr<AdjointPlan> build_plan(const std::vector<GateDesc>& tmpl,
     }
     plan->psi = plan->states->psi.get();
     plan->lam = plan->states->lam.get();
-    plan->ham.upload(h, n);
+    plan->ham.upload(*hh, n);
     plan->plan_tiles();
-    plan->d_cs.ensure(sizeof(double2) * std::max<uint64_t>(1, np) * R);
-    plan->d_csi.ensure(sizeof(double2) * std::max<uint64_t>(1, np) * R);
+    plan->d_cs.ensure(sizeof(double2) * std::max<uint64_t>(1, plan->np_all) * R);
+    plan->d_csi.ensure(sizeof(double2) * std::max<uint64_t>(1, plan->np_all) * R);
     plan->d_part.ensure(sizeof(double) * 64 * R);
     plan->d_energy.ensure(sizeof(double) * R);
-    plan->d_grad.ensure(sizeof(double) * std::max<uint64_t>(1, np) * R);
+    plan->d_grad.ensure(sizeof(double) * std::max<uint64_t>(1, plan->np_all) * R);
     return plan;
 }
 
@@ -644,8 +795,15 @@ void adjoint_batched(const lqcs_parametric_circuit* pc, const Hamiltonian& h,
     AdjointPlan& plan = *held;   // alive although another call may drop it from the list
     std::lock_guard<std::mutex> busy(plan.states->mu);
     const uint32_t R = plan.R;
-    std::vector<double2> cs(np * R), csi(np * R);
-    std::vector<double> h_energy(R), h_grad(np * R);
+    const uint64_t rows = plan.np_all;
+    std::vector<double2> cs(rows * R), csi(rows * R);
+    std::vector<double> h_energy(R), h_grad(rows * R);
+    for (uint64_t p = np; p < rows; ++p)
+        for (uint32_t b = 0; b < R; ++b) {
+            const double hh = plan.fixed[p - np] / 2;
+            cs[p * R + b] = make_double2(std::cos(hh), std::sin(hh));
+            csi[p * R + b] = make_double2(std::cos(hh), -std::sin(hh));
+        }
     for (uint64_t b0 = 0; b0 < batch; b0 += R) {
         const uint32_t nb = static_cast<uint32_t>(std::min<uint64_t>(R, batch - b0));
         // (cos, sin) of theta/2 per parameter and set; layout [param][set]
@@ -656,23 +814,23 @@ void adjoint_batched(const lqcs_parametric_circuit* pc, const Hamiltonian& h,
                 csi[p * R + b] = make_double2(std::cos(hh), -std::sin(hh));
             }
         }
-        if (np) {
-            cuda_check(cudaMemcpyAsync(plan.d_cs.ptr, cs.data(), sizeof(double2) * np * R,
+        if (rows) {
+            cuda_check(cudaMemcpyAsync(plan.d_cs.ptr, cs.data(), sizeof(double2) * rows * R,
                                        cudaMemcpyHostToDevice, plan.stream), "H2D");
-            cuda_check(cudaMemcpyAsync(plan.d_csi.ptr, csi.data(), sizeof(double2) * np * R,
+            cuda_check(cudaMemcpyAsync(plan.d_csi.ptr, csi.data(), sizeof(double2) * rows * R,
                                        cudaMemcpyHostToDevice, plan.stream), "H2D");
         }
         plan.run(nb, grad_out != nullptr);
         cuda_check(cudaMemcpyAsync(h_energy.data(), plan.d_energy.ptr, sizeof(double) * nb,
                                    cudaMemcpyDeviceToHost, plan.stream), "D2H energies");
         if (np && grad_out)
-            cuda_check(cudaMemcpyAsync(h_grad.data(), plan.d_grad.ptr, sizeof(double) * np * nb,
+            cuda_check(cudaMemcpyAsync(h_grad.data(), plan.d_grad.ptr, sizeof(double) * rows * nb,
                                        cudaMemcpyDeviceToHost, plan.stream), "D2H gradients");
         cuda_check(cudaStreamSynchronize(plan.stream), "adjoint");
         for (uint32_t b = 0; b < nb; ++b) {
             if (energy_out) energy_out[b0 + b] = h_energy[b];
             if (grad_out)
-                std::copy(h_grad.begin() + b * np, h_grad.begin() + (b + 1) * np,
+                std::copy(h_grad.begin() + b * rows, h_grad.begin() + b * rows + np,
                           grad_out + (b0 + b) * np);
         }
     }
@@ -834,22 +992,22 @@ void adjoint_batched_multi(uint64_t n_problems, const lqcs_parametric_circuit* c
     std::vector<std::vector<double2>> tabs(2 * n_problems);
     for (uint64_t p = 0; p < n_problems; ++p) {
         const AdjointPlan& pl = *mp->plans[p];
-        const uint64_t np = pl.np, R = pl.R;
+        const uint64_t np = pl.np, rows = pl.np_all, R = pl.R;
         std::vector<double2>& cs = tabs[2 * p];
         std::vector<double2>& csi = tabs[2 * p + 1];
-        cs.resize(np * R);
-        csi.resize(np * R);
-        for (uint64_t k = 0; k < np; ++k) {
+        cs.resize(rows * R);
+        csi.resize(rows * R);
+        for (uint64_t k = 0; k < rows; ++k) {
             for (uint64_t b = 0; b < R; ++b) {
-                const double hh = params[p][b * np + k] / 2;
+                const double hh = (k < np ? params[p][b * np + k] : pl.fixed[k - np]) / 2;
                 cs[k * R + b] = make_double2(std::cos(hh), std::sin(hh));
                 csi[k * R + b] = make_double2(std::cos(hh), -std::sin(hh));
             }
         }
-        if (np) {
-            cuda_check(cudaMemcpyAsync(pl.d_cs.ptr, cs.data(), sizeof(double2) * np * R,
+        if (rows) {
+            cuda_check(cudaMemcpyAsync(pl.d_cs.ptr, cs.data(), sizeof(double2) * rows * R,
                                        cudaMemcpyHostToDevice, mp->origin), "H2D");
-            cuda_check(cudaMemcpyAsync(pl.d_csi.ptr, csi.data(), sizeof(double2) * np * R,
+            cuda_check(cudaMemcpyAsync(pl.d_csi.ptr, csi.data(), sizeof(double2) * rows * R,
                                        cudaMemcpyHostToDevice, mp->origin), "H2D");
         }
     }
@@ -860,8 +1018,9 @@ void adjoint_batched_multi(uint64_t n_problems, const lqcs_parametric_circuit* c
             cuda_check(cudaMemcpyAsync(energy_out[p], pl.d_energy.ptr, sizeof(double) * pl.R,
                                        cudaMemcpyDeviceToHost, mp->origin), "D2H energies");
         if (grad_out && grad_out[p] && pl.np)
-            cuda_check(cudaMemcpyAsync(grad_out[p], pl.d_grad.ptr, sizeof(double) * pl.np * pl.R,
-                                       cudaMemcpyDeviceToHost, mp->origin), "D2H gradients");
+            cuda_check(cudaMemcpy2DAsync(grad_out[p], sizeof(double) * pl.np, pl.d_grad.ptr,
+                                         sizeof(double) * pl.np_all, sizeof(double) * pl.np, pl.R,
+                                         cudaMemcpyDeviceToHost, mp->origin), "D2H gradients");
     }
     cuda_check(cudaStreamSynchronize(mp->origin), "adjoint_gradient_multi");
 }

@@ -142,9 +142,10 @@ void launch_move_to_zero(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t
 // ---------------------------------------------------------------- Hamiltonian
 // out = sum_t c_t P_t in (per state of a batch); terms in device memory.
 struct PauliTermDev {
-    uint64_t x;
     uint64_t zy;
-    double2 coeff;   // c_t * i^{n_y}
+    double w;        // c_t i^{n_y} (-1)^{popcount(x & zy)} = w, or i w with imag
+    uint32_t x_lo;   // x below ham_tile_bits
+    uint32_t imag;
 };
 // Tile bits of the Hamiltonian apply.  Its terms come grouped by x >> ham_tile_bits(n) (the
 // groups in any order, terms of a group contiguous); d_groups = {G, G group keys, G + 1 term
