@@ -312,6 +312,142 @@ __global__ void __launch_bounds__(256) k_adj_grad(const double* __restrict__ par
     if (lane == 0) grad[static_cast<uint64_t>(b) * np + p.rot[k].param] = v;
 }
 
+// ---------------------------------------------------------------- expectations
+// Statevector::expectation_value (src/backend/statevector.cpp:39-78):
+// <P> = Re( i^{n_y} sum_i s_i a_i conj(a_{i ^ x}) ), s_i = (-1)^{popcount(i & zy)}.
+// The terms of i and i ^ x are conjugate up to (-1)^{n_y} (n_y = popcount(x & zy) mod 2), so a
+// pair gives twice a real (n_y even) or imaginary (odd) part.
+
+// Sum of s_u |a_u|^2, or of s_u times that part over the pairs of register bit RB.
+template <int E, int RB, bool ODD>
+__device__ __forceinline__ double pair_sum(const double2 (&v)[E], const Signs& sg) {
+    double acc = 0.0;
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        if ((u >> RB) & 1) continue;
+        const double2 a = v[u], b = v[u | (1 << RB)];
+        const double r = ODD ? fma(a.y, b.x, -a.x * b.y) : fma(a.x, b.x, a.y * b.y);
+        acc += toggle(r, sg(u));
+    }
+    return acc;
+}
+template <int RB>
+__device__ __forceinline__ double term_sum(const double2 (&v)[16], uint32_t n_y, const Signs& sg) {
+    return (n_y & 1u) ? pair_sum<16, RB, true>(v, sg) : pair_sum<16, RB, false>(v, sg);
+}
+
+// The factor of a term's sum: 2 i^{n_y} (n_y even) or 2 i^{n_y + 1} (odd); 1 without pairs.
+__device__ __forceinline__ double term_factor(bool pairs, uint32_t n_y) {
+    if (!pairs) return 1.0;
+    return (n_y == 0u || n_y == 3u) ? 2.0 : -2.0;
+}
+
+// Persistent CTAs over the tiles; each thread keeps a sum per term (in shared memory), added up
+// tile after tile, and the block's sums go out once.  HBM-bound: 16 bytes per amplitude for up
+// to nine independent x masks, where a launch per x mask read the state for each.
+__global__ void __launch_bounds__(256, 2) k_expect_pass(const double2* __restrict__ s,
+                                                        uint32_t n_tiles,
+                                                        const __grid_constant__ AdjPass p,
+                                                        double* __restrict__ partials) {
+    constexpr int M = kExpectTileBits, TB = M - 4, E = 16;
+    constexpr uint32_t T = 1u << TB;
+    extern __shared__ __align__(16) double2 tile[];
+    double* sums = reinterpret_cast<double*>(tile + (1u << M));
+    for (uint32_t k = 0; k < p.n_rots; ++k) sums[k * T + threadIdx.x] = 0.0;
+    const uint64_t off = thread_offset<TB>(p, 0);
+    for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        const uint64_t base = tile_base(p, t);
+        double2 v[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) v[u] = __ldcs(s + (base ^ off ^ reg_offset<4>(p, 0, u)));
+        uint32_t cur = 0;
+        for (uint32_t k = 0; k < p.n_rots; ++k) {
+            const AdjRot& r = p.rot[k];
+            if (cur != r.layout) {
+                __syncthreads();   // the previous remap's reads
+                const uint32_t a = thread_slot<TB>(p.lay[cur]);
+#pragma unroll
+                for (int u = 0; u < E; ++u) tile[a ^ reg_slot<4>(p.lay[cur], u)] = v[u];
+                cur = r.layout;
+                __syncthreads();
+                const uint32_t b = thread_slot<TB>(p.lay[cur]);
+#pragma unroll
+                for (int u = 0; u < E; ++u) v[u] = tile[b ^ reg_slot<4>(p.lay[cur], u)];
+            }
+            const Signs sg(__popcll(base & r.zy) + __popc(threadIdx.x & r.tz), r.rz);
+            double g;
+            switch (r.rbit) {
+                case 0: g = term_sum<0>(v, r.n_y, sg); break;
+                case 1: g = term_sum<1>(v, r.n_y, sg); break;
+                case 2: g = term_sum<2>(v, r.n_y, sg); break;
+                case 3: g = term_sum<3>(v, r.n_y, sg); break;
+                default:
+                    g = 0.0;
+#pragma unroll
+                    for (int u = 0; u < E; ++u) g += toggle(fma(v[u].x, v[u].x, v[u].y * v[u].y), sg(u));
+            }
+            sums[k * T + threadIdx.x] += g;
+        }
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = threadIdx.x >> 5; k < p.n_rots; k += T / 32) {
+        double g = 0.0;
+#pragma unroll
+        for (uint32_t j = 0; j < T / 32; ++j) g += sums[k * T + j * 32 + lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+        const AdjRot& r = p.rot[k];
+        if (lane == 0)
+            partials[static_cast<uint64_t>(r.param) * gridDim.x + blockIdx.x] =
+                term_factor(r.rbit != kAdjDiag, r.n_y) * g;
+    }
+}
+
+// out[t] = the sum of term t's partials: one warp, lanes over the blocks in order, a butterfly.
+__global__ void __launch_bounds__(256) k_expect_sum(const double* __restrict__ partials, uint32_t blocks,
+                                                    uint32_t n_terms, double* __restrict__ out) {
+    const uint32_t t = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (t >= n_terms) return;   // whole warps
+    double g = 0.0;
+    for (uint32_t b = lane; b < blocks; b += 32) g += partials[static_cast<uint64_t>(t) * blocks + b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    if (lane == 0) out[t] = g;
+}
+
+// States of up to 2^14 amplitudes: one block per term, the state from L2.
+__global__ void __launch_bounds__(256) k_expect_small(const double2* __restrict__ s, uint64_t len,
+                                                      const AdjRotation* __restrict__ terms,
+                                                      double* __restrict__ out) {
+    const AdjRotation r = terms[blockIdx.x];
+    double g = 0.0;
+    if (r.x == 0) {
+        for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) {
+            const double2 a = __ldg(s + i);
+            g += toggle(fma(a.x, a.x, a.y * a.y), static_cast<uint32_t>(__popcll(i & r.zy)) << 31);
+        }
+    } else {
+        const unsigned hb = 63u - static_cast<unsigned>(__clzll(static_cast<long long>(r.x)));
+        for (uint64_t q = threadIdx.x; q < len / 2; q += blockDim.x) {
+            const uint64_t i = insert_zero_bit(q, hb);
+            const double2 a = __ldg(s + i), b = __ldg(s + (i ^ r.x));
+            const double z = (r.n_y & 1u) ? fma(a.y, b.x, -a.x * b.y) : fma(a.x, b.x, a.y * b.y);
+            g += toggle(z, static_cast<uint32_t>(__popcll(i & r.zy)) << 31);
+        }
+    }
+    __shared__ double red[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = g;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += red[w];
+        out[blockIdx.x] = term_factor(r.x != 0, r.n_y & 3u) * t;
+    }
+}
+
 void check_pass(const AdjPass& p, uint32_t n, uint32_t regs) {
     if (p.m > n || p.m < kAdjMinBits || p.m > kAdjMaxBits || p.regs != regs ||
         p.n_rots > kAdjMaxRots || p.n_rots == 0 || p.n_layouts > kAdjMaxLayouts)
@@ -340,6 +476,33 @@ void bwd(const LaunchCtx& ctx, double2* psi, double2* lam, uint32_t n, uint32_t 
 }
 
 }  // namespace
+
+uint32_t expect_blocks(const LaunchCtx& ctx, uint32_t n) {
+    return std::min<uint32_t>(1u << (n - kExpectTileBits), static_cast<uint32_t>(ctx.num_sms) * 2);
+}
+
+void launch_expect_pass(const LaunchCtx& ctx, const double2* st, uint32_t n, const AdjPass& p,
+                        double* d_partials) {
+    check_pass(p, n, 4);
+    if (p.m != kExpectTileBits || p.n_rots > kExpectTerms) throw std::logic_error("expectation pass: unsupported shape");
+    const size_t smem = (sizeof(double2) << kExpectTileBits) + sizeof(double) * p.n_rots * (1u << (kExpectTileBits - 4));
+    cuda_check_launch_attr(cudaFuncSetAttribute(k_expect_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(smem)));
+    k_expect_pass<<<expect_blocks(ctx, n), 256, smem, ctx.stream>>>(st, 1u << (n - kExpectTileBits), p, d_partials);
+    check_launch("expectation pass");
+}
+
+void launch_expect_sum(const LaunchCtx& ctx, uint32_t n, uint32_t n_terms, const double* d_partials,
+                       double* d_out) {
+    k_expect_sum<<<(n_terms + 7) / 8, 256, 0, ctx.stream>>>(d_partials, expect_blocks(ctx, n), n_terms, d_out);
+    check_launch("expectation sum");
+}
+
+void launch_expect_small(const LaunchCtx& ctx, const double2* st, uint32_t n,
+                         const AdjRotation* d_terms, uint32_t n_terms, double* d_out) {
+    k_expect_small<<<n_terms, 256, 0, ctx.stream>>>(st, uint64_t{1} << n, d_terms, d_out);
+    check_launch("expectation");
+}
 
 void launch_adj_fwd(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t nb, const AdjPass& p,
                     const double2* d_cs, uint32_t R) {

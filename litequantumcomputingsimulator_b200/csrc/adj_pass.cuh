@@ -51,9 +51,22 @@ struct AdjRotation {
 };
 
 // Passes over rotations in the order given (a rotation may move ahead of others it commutes
-// with), on an n-qubit register, m = min(n, `bits`) >= kAdjMinBits.
+// with; of all with any_order), on an n-qubit register, m = min(n, `bits`) >= kAdjMinBits.
 std::vector<AdjPass> plan_adjoint_passes(const std::vector<AdjRotation>& rots, uint32_t n,
-                                         uint32_t bits, uint32_t regs);
+                                         uint32_t bits, uint32_t regs, bool any_order = false,
+                                         uint32_t most = kAdjMaxRots);
+
+// Pauli expectations <psi|P|psi> of terms i^n_y X^x Z^zy on the same tiles: a pass reads the state
+// once for every term whose x lies in its tiles' subspace.  param: the term's place in d_out.
+constexpr uint32_t kExpectTileBits = 12, kExpectTerms = 20;   // per pass
+constexpr uint32_t kExpectSmall = 14;                         // to here: a block per term
+uint32_t expect_blocks(const LaunchCtx& ctx, uint32_t n);      // partials per term, n > kExpectSmall
+void launch_expect_pass(const LaunchCtx& ctx, const double2* st, uint32_t n, const AdjPass& p,
+                        double* d_partials);
+void launch_expect_sum(const LaunchCtx& ctx, uint32_t n, uint32_t n_terms, const double* d_partials,
+                       double* d_out);
+void launch_expect_small(const LaunchCtx& ctx, const double2* st, uint32_t n,
+                         const AdjRotation* d_terms, uint32_t n_terms, double* d_out);
 
 void launch_adj_fwd(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t nb, const AdjPass& p,
                     const double2* d_cs, uint32_t R);

@@ -136,7 +136,8 @@ AdjPass make_pass(const std::vector<AdjRotation>& rots, Span space, uint32_t n, 
 }  // namespace
 
 std::vector<AdjPass> plan_adjoint_passes(const std::vector<AdjRotation>& rots, uint32_t n,
-                                         uint32_t bits, uint32_t regs) {
+                                         uint32_t bits, uint32_t regs, bool any_order,
+                                         uint32_t most) {
     const uint32_t m = std::min(n, std::min(bits, kAdjMaxBits));
     if (m < kAdjMinBits) throw std::logic_error("adjoint pass: too few qubits");
     std::vector<AdjPass> out;
@@ -147,9 +148,9 @@ std::vector<AdjPass> plan_adjoint_passes(const std::vector<AdjRotation>& rots, u
         std::vector<AdjRotation> cur, rest;
         uint32_t layouts = 1, in_layout = 0;   // an upper bound on the layouts taken so far
         for (const AdjRotation& r : pend) {
-            bool ok = cur.size() < kAdjMaxRots && layouts < kAdjMaxLayouts &&
+            bool ok = cur.size() < most && layouts < kAdjMaxLayouts &&
                       (space.v.size() < m || space.contains(r.x));
-            for (size_t k = 0; ok && k < rest.size(); ++k) ok = commute(r, rest[k]);
+            for (size_t k = 0; !any_order && ok && k < rest.size(); ++k) ok = commute(r, rest[k]);
             if (!ok) {
                 rest.push_back(r);
                 continue;

@@ -1,6 +1,7 @@
 // engine.cpp — device runtime: state handles, programs, run paths, expectations.
 #include "engine.hpp"
 
+#include "adj_pass.cuh"
 #include "costmodel.hpp"
 
 #include <algorithm>
@@ -1071,36 +1072,34 @@ double state_norm2(lqcs_state& st) {
 std::vector<double> expectation_terms(lqcs_state& st, const std::vector<PauliMasks>& terms) {
     std::vector<double> vals(terms.size(), 0.0);
     if (terms.empty()) return vals;
-    // group terms by x mask (one read of a_i, a_{i^x} per group of up to 8 terms)
-    std::map<uint64_t, std::vector<size_t>> groups;
-    for (size_t t = 0; t < terms.size(); ++t) groups[terms[t].x].push_back(t);
-    double* part = st.partials(2 * kMaxTermsPerPass + 1);
-    const size_t part_len = (kMaxReduceBlocks + 1) * 2 * kMaxTermsPerPass * 2;
-    DeviceBuffer d_out;
-    d_out.ensure(sizeof(double) * terms.size());
-    double* out = d_out.as<double>();
-    std::vector<size_t> order;
-    for (auto& [x, idx] : groups) {
-        for (size_t s = 0; s < idx.size(); s += kMaxTermsPerPass) {
-            const uint32_t cnt = static_cast<uint32_t>(std::min<size_t>(kMaxTermsPerPass, idx.size() - s));
-            uint64_t zy[kMaxTermsPerPass];
-            uint32_t ny[kMaxTermsPerPass];
-            for (uint32_t c = 0; c < cnt; ++c) {
-                zy[c] = terms[idx[s + c]].zy;
-                ny[c] = terms[idx[s + c]].n_y;
-                order.push_back(idx[s + c]);
-            }
-            launch_expect_xgroup(st.ctx, st.d(), st.n, x, zy, ny, cnt, part,
-                                 out + (order.size() - cnt));
-            (void)part_len;
-        }
+    const uint32_t count = static_cast<uint32_t>(terms.size());
+    std::vector<AdjRotation> list;
+    for (uint32_t t = 0; t < count; ++t) list.push_back({terms[t].x, terms[t].zy, terms[t].n_y & 3u, t});
+    if (st.n <= kExpectSmall) {
+        st.scratch.ensure((sizeof(AdjRotation) + sizeof(double)) * count);
+        AdjRotation* d_terms = st.scratch.as<AdjRotation>();
+        double* d_out = reinterpret_cast<double*>(d_terms + count);
+        cuda_check(cudaMemcpyAsync(d_terms, list.data(), sizeof(AdjRotation) * count,
+                                   cudaMemcpyHostToDevice, st.stream), "H2D terms");
+        launch_expect_small(st.ctx, st.d(), st.n, d_terms, count, d_out);
+        cuda_check(cudaMemcpyAsync(vals.data(), d_out, sizeof(double) * count,
+                                   cudaMemcpyDeviceToHost, st.stream), "D2H expectations");
+        st.sync();
+        return vals;
     }
-    std::vector<double> packed(terms.size());
-    cuda_check(cudaMemcpyAsync(packed.data(), out, sizeof(double) * terms.size(),
-                               cudaMemcpyDeviceToHost, st.stream),
-               "D2H expectations");
+    // terms of one x mask side by side: they share a layout
+    std::stable_sort(list.begin(), list.end(),
+                     [](const AdjRotation& a, const AdjRotation& b) { return a.x < b.x; });
+    const uint32_t blocks = expect_blocks(st.ctx, st.n);
+    st.scratch.ensure(sizeof(double) * count * (size_t{blocks} + 1));
+    double* part = st.scratch.as<double>();
+    double* d_out = part + static_cast<size_t>(count) * blocks;
+    for (const AdjPass& p : plan_adjoint_passes(list, st.n, kExpectTileBits, 4, true, kExpectTerms))
+        launch_expect_pass(st.ctx, st.d(), st.n, p, part);
+    launch_expect_sum(st.ctx, st.n, count, part, d_out);
+    cuda_check(cudaMemcpyAsync(vals.data(), d_out, sizeof(double) * count, cudaMemcpyDeviceToHost,
+                               st.stream), "D2H expectations");
     st.sync();
-    for (size_t k = 0; k < order.size(); ++k) vals[order[k]] = packed[k];
     return vals;
 }
 

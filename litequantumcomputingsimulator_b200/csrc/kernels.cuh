@@ -102,13 +102,6 @@ void launch_rdm1(const LaunchCtx& ctx, const double2* st, uint32_t n, uint32_t q
 // sum_pairs ||K (a0, a1)||^2 -> d_out[0]
 void launch_kraus_prob(const LaunchCtx& ctx, const double2* st, uint32_t n, uint32_t q,
                        const double2 k[4], double* d_partials, double* d_out);
-// Pauli expectation: d_out[t] = Re(i^{n_y[t]} sum_i sign_t(i) a_i conj(a_{i^x})) for
-// n_terms terms that share the x mask (zy, n_y: host arrays of n_terms entries).
-// n_terms <= kMaxTermsPerPass; d_partials holds (kMaxReduceBlocks + 1) * 16 doubles.
-constexpr uint32_t kMaxTermsPerPass = 8;
-void launch_expect_xgroup(const LaunchCtx& ctx, const double2* st, uint32_t n, uint64_t x,
-                          const uint64_t* zy, const uint32_t* n_y, uint32_t n_terms,
-                          double* d_partials, double* d_out);
 // probabilities p[i] = |a_i|^2 (rounded like std::norm)
 void launch_probabilities(const LaunchCtx& ctx, const double2* st, uint32_t n, double* d_p);
 

@@ -191,97 +191,6 @@ void launch_kraus_prob(const LaunchCtx& ctx, const double2* st, uint32_t n, uint
     finalize<1>(ctx, d_partials, nb, d_out);
 }
 
-// ---------------------------------------------------------------- Pauli expectation
-// Statevector::expectation_value (src/backend/statevector.cpp:39-78):
-// <P> = Re( i^{n_y} sum_i (-1)^{popcount(i & zy)} a_i conj(a_{i ^ x}) ).
-// Terms sharing an x mask share the one read of a_i and a_{i ^ x}.
-struct PExpect {
-    uint64_t x;
-    uint64_t len;
-    uint32_t n_terms;
-    uint32_t n_y[kMaxTermsPerPass];
-    uint64_t zy[kMaxTermsPerPass];
-};
-
-__global__ void __launch_bounds__(kReduceThreads) k_expect(const double2* __restrict__ s,
-                                                           PExpect p, double* partials) {
-    double v[2 * kMaxTermsPerPass];
-#pragma unroll
-    for (int k = 0; k < static_cast<int>(2 * kMaxTermsPerPass); ++k) v[k] = 0.0;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    if (p.x == 0) {
-        for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-             i < p.len; i += stride) {
-            const double2 a = __ldg(s + i);
-            const double wr = a.x * a.x + a.y * a.y;
-#pragma unroll
-            for (int t = 0; t < static_cast<int>(kMaxTermsPerPass); ++t) {
-                if (t < static_cast<int>(p.n_terms)) v[2 * t] += parity_sign(i & p.zy[t]) * wr;
-            }
-        }
-    } else {
-        // each pair (i, i ^ x) once: the term at i ^ x is the conjugate of the one at i, with
-        // its own sign, so every amplitude is read once
-        const unsigned hb = 63u - static_cast<unsigned>(__clzll(p.x));
-        for (uint64_t g = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-             g < p.len / 2; g += stride) {
-            const uint64_t i = insert_zero_bit(g, hb), j = i ^ p.x;
-            const double2 a = __ldg(s + i), b = __ldg(s + j);
-            // a * conj(b) at i; b * conj(a) = its conjugate at j
-            const double wr = a.x * b.x + a.y * b.y;
-            const double wi = a.y * b.x - a.x * b.y;
-#pragma unroll
-            for (int t = 0; t < static_cast<int>(kMaxTermsPerPass); ++t) {
-                if (t < static_cast<int>(p.n_terms)) {
-                    const double si = parity_sign(i & p.zy[t]), sj = parity_sign(j & p.zy[t]);
-                    v[2 * t] += (si + sj) * wr;
-                    v[2 * t + 1] += (si - sj) * wi;
-                }
-            }
-        }
-    }
-    block_sum_store<2 * kMaxTermsPerPass>(v, partials + blockIdx.x, gridDim.x);
-}
-
-__global__ void k_expect_combine(const double* __restrict__ sums, PExpect p,
-                                 double* __restrict__ out) {
-    const uint32_t t = threadIdx.x;
-    if (t >= p.n_terms) return;
-    const double re = sums[2 * t], im = sums[2 * t + 1];
-    // Re(i^{n_y} (re + i im))
-    double r;
-    switch (p.n_y[t] & 3u) {
-        case 0: r = re; break;
-        case 1: r = -im; break;
-        case 2: r = -re; break;
-        default: r = im; break;
-    }
-    out[t] = r;
-}
-
-void launch_expect_xgroup(const LaunchCtx& ctx, const double2* st, uint32_t n, uint64_t x,
-                          const uint64_t* zy, const uint32_t* n_y, uint32_t n_terms,
-                          double* d_partials, double* d_out) {
-    if (n_terms == 0 || n_terms > kMaxTermsPerPass)
-        throw std::logic_error("launch_expect_xgroup: bad term count");
-    PExpect p{};
-    p.x = x;
-    p.len = uint64_t{1} << n;
-    p.n_terms = n_terms;
-    for (uint32_t t = 0; t < n_terms; ++t) {
-        p.zy[t] = zy[t];
-        p.n_y[t] = n_y[t];
-    }
-    const uint32_t nb = reduce_grid(ctx, p.len);
-    k_expect<<<nb, kReduceThreads, 0, ctx.stream>>>(st, p, d_partials);
-    check_launch("expect");
-    // reuse the tail of the partial buffer for the 2*kMaxTermsPerPass sums
-    double* sums = d_partials + static_cast<uint64_t>(nb) * 2 * kMaxTermsPerPass;
-    finalize<2 * kMaxTermsPerPass>(ctx, d_partials, nb, sums);
-    k_expect_combine<<<1, 32, 0, ctx.stream>>>(sums, p, d_out);
-    check_launch("expect_combine");
-}
-
 // ---------------------------------------------------------------- probabilities
 // Statevector::probabilities (src/backend/statevector.cpp:33-37)
 __global__ void k_probs(const double2* __restrict__ s, uint64_t len, double* __restrict__ p) {
