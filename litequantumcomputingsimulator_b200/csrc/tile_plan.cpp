@@ -12,6 +12,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <deque>
+#include <map>
+#include <string>
 #include <tuple>
 
 #include "tile_plan.hpp"
@@ -213,6 +215,14 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
             continue;
         }
         if (!g.slot && plain_1q(g)) {
+            if (role[i] == kDiag1) {   // a damping factor: between two gates it would leave no
+                const std::vector<cd> m = g.base_matrix();   // rotation form, in a table it is free
+                if (std::abs(std::abs(m[0]) - std::abs(m[3])) > 1e-12) {
+                    flush(g.qubits[0]);
+                    push(g);
+                    continue;
+                }
+            }
             multiply(g.qubits[0], g, g.src);
             continue;
         }
@@ -716,7 +726,9 @@ static void merge_diagonal_runs(std::vector<LocalOp>& ops, uint32_t max_bits, bo
 // block on it without controls (the ops in between do not touch the qubit, so they commute
 // with it): the block's matrix absorbs it at no extra cost per amplitude and one operation
 // disappears.  A noise slot (per-state matrix) folds too: the block becomes per-state.
-static void fold_single_qubit_ops(std::vector<LocalOp>& ops, uint32_t max_select) {
+// In rotation form a diagonal stays out of one-qubit blocks: it is free in a table, and with a
+// damping factor a block would have no rotation form any more (16 flops per amplitude, not 4).
+static void fold_single_qubit_ops(std::vector<LocalOp>& ops, uint32_t max_select, bool rot) {
     std::vector<char> dead(ops.size(), 0);
     for (size_t i = 0; i < ops.size(); ++i) {
         // a phase on one tile bit (such as K0 of amplitude damping) folds as the diagonal
@@ -741,7 +753,8 @@ static void fold_single_qubit_ops(std::vector<LocalOp>& ops, uint32_t max_select
                                  std::find(q.lt.begin(), q.lt.end(), a) != q.lt.end();
             if (!touches) continue;
             const auto it = std::find(q.lt.begin(), q.lt.end(), a);
-            if (q.kind == kTileDense && it != q.lt.end() && !q.lmask && !q.gcmask) {
+            if (q.kind == kTileDense && it != q.lt.end() && !q.lmask && !q.gcmask &&
+                !(rot && q.lt.size() == 1 && p.kind == kTileDiag)) {
                 std::vector<uint32_t> sel = q.sel;
                 for (uint32_t s : p.sel)
                     if (std::find(sel.begin(), sel.end(), s) == sel.end()) sel.push_back(s);
@@ -762,7 +775,8 @@ static void fold_single_qubit_ops(std::vector<LocalOp>& ops, uint32_t max_select
                                  std::find(q.lt.begin(), q.lt.end(), a) != q.lt.end();
             if (!touches) continue;
             const auto it = std::find(q.lt.begin(), q.lt.end(), a);
-            if (q.kind == kTileDense && it != q.lt.end() && !q.lmask && !q.gcmask) {
+            if (q.kind == kTileDense && it != q.lt.end() && !q.lmask && !q.gcmask &&
+                !(rot && q.lt.size() == 1 && p.kind == kTileDiag)) {
                 std::vector<uint32_t> sel = q.sel;
                 for (uint32_t s : p.sel)
                     if (std::find(sel.begin(), sel.end(), s) == sel.end()) sel.push_back(s);
@@ -1082,7 +1096,7 @@ std::vector<LocalOp> pass_local_ops(const PlanItem& item, const std::vector<Gate
     for (Open& b : open) emit_block(b);
     // one-qubit ops first go into the dense blocks on their qubits (free); the diagonal
     // work left over then merges into tables
-    fold_single_qubit_ops(out, max_select);
+    fold_single_qubit_ops(out, max_select, rot);
     if (rot) split_rotations(out);
     else merge_diagonal_runs(out, max_diag, dyn_terms);
     if (store_qubits) {   // qubit each tile bit holds at the end of the pass
@@ -2144,7 +2158,26 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     const size_t n_mat = mats.size();
     // every further state: same records, its own slot matrices
     if (state_slots) {
+        // (states with the same matrices in all of the pass's slots, most often no error at all,
+        // share the work)
+        std::map<std::string, size_t> known;   // slot matrices -> the state lowered for them
+        auto key_of = [&](size_t b) {
+            std::string k;
+            for (uint32_t gi : item.gates)
+                if (gates[gi].slot)
+                    k.append(reinterpret_cast<const char*>((*state_slots)[b][gates[gi].slot_id].data()),
+                             sizeof(std::array<cd, 4>));
+            return k;
+        };
+        known.emplace(key_of(0), 0);
         for (size_t b = 1; b < state_slots->size(); ++b) {
+            const auto [same, fresh] = known.emplace(key_of(b), b);
+            if (!fresh) {
+                mats.resize(mats.size() + n_mat);
+                std::copy_n(mats.begin() + static_cast<long>(same->second * n_mat), n_mat,
+                            mats.end() - static_cast<long>(n_mat));
+                continue;
+            }
             std::vector<uint32_t> store_b;
             const std::vector<LocalOp> ob = pass_local_ops(item, gates, cfg, max_select,
                                                            &(*state_slots)[b], kRegMaxDiag, true,

@@ -173,9 +173,8 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
     mats.ensure(sizeof(double2) * R * 4);
     flag.ensure(sizeof(int) * R);
     scale.ensure(sizeof(double) * R);
-    dregs.ensure(sizeof(uint64_t) * R);
-    TrajScratch scr{part.as<double>(), mats.as<double2>(), flag.as<int>(), scale.as<double>(),
-                    dregs.as<uint64_t>()};
+    dregs.ensure(sizeof(uint64_t) * f.shots);   // of every batch: read back once, at the end
+    cuda_check(cudaMemsetAsync(dregs.ptr, 0, sizeof(uint64_t) * f.shots, cs), "memset");
     const Kraus ident{cd{1, 0}, cd{0, 0}, cd{0, 0}, cd{1, 0}};
     // Terminal measurements (nothing but Measures of distinct qubits up to the end) need no
     // collapse: each outcome follows from the amplitudes consistent with the earlier ones.
@@ -190,17 +189,26 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
     DeviceBuffer d_vals;
     d_vals.ensure(sizeof(uint64_t) * R);
 
+    // The host lowers a batch while the device still runs the one before: what the device reads
+    // stays alive until the end, or until 256 MiB of it have gathered.
+    struct Held {
+        std::vector<Program> programs;
+        std::vector<DeviceBuffer> buffers;
+    };
+    std::vector<Held> held;
+    size_t held_bytes = 0;
     for (uint64_t first = 0; first < f.shots;) {   // first: batch start position in `order`
         const uint32_t nb = static_cast<uint32_t>(
             first < n_clean ? std::min<uint64_t>(R, n_clean - first)
                             : std::min<uint64_t>(R_dirty, f.shots - first));
         auto shot = [&](uint32_t b) { return order[first + b]; };
         launch_set_basis(ctx, st->d(), n, nb, 0);
-        cuda_check(cudaMemsetAsync(dregs.ptr, 0, sizeof(uint64_t) * nb, cs), "memset");
+        TrajScratch scr{part.as<double>(), mats.as<double2>(), flag.as<int>(), scale.as<double>(),
+                        dregs.as<uint64_t>() + first};
         cuda_check(cudaMemsetAsync(d_vals.ptr, 0, sizeof(uint64_t) * nb, cs), "memset");
         BitList tail_fixed{};
-        std::vector<Program> keep;          // alive until the batch is done
-        std::vector<DeviceBuffer> bufs;
+        std::vector<Program>& keep = held.emplace_back().programs;
+        std::vector<DeviceBuffer>& bufs = held.back().buffers;
         std::vector<GateDesc> seg;
         std::vector<std::vector<Kraus>> slots(nb);
         auto upload = [&](const void* src, size_t bytes) {
@@ -329,11 +337,20 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
             }
         }
         flush();
-        cuda_check(cudaMemcpyAsync(regs_perm.data() + first, dregs.ptr, sizeof(uint64_t) * nb,
-                                   cudaMemcpyDeviceToHost, cs), "D2H registers");
-        cuda_check(cudaStreamSynchronize(cs), "trajectory batch");
+        for (const Program& p : keep)
+            held_bytes += p.d_mats.bytes + p.d_u32.bytes + p.d_reg_ops.bytes + p.d_reg_layouts.bytes +
+                          p.d_reg_mats.bytes + p.d_tile_ops.bytes + p.d_tile_mats.bytes;
+        for (const DeviceBuffer& b : bufs) held_bytes += b.bytes;
+        if (held_bytes > (size_t{256} << 20)) {
+            cuda_check(cudaStreamSynchronize(cs), "trajectory batch");
+            held.clear();
+            held_bytes = 0;
+        }
         first += nb;
     }
+    cuda_check(cudaMemcpyAsync(regs_perm.data(), dregs.ptr, sizeof(uint64_t) * f.shots,
+                               cudaMemcpyDeviceToHost, cs), "D2H registers");
+    cuda_check(cudaStreamSynchronize(cs), "trajectories");
     for (uint64_t p = 0; p < f.shots; ++p) regs[order[p]] = regs_perm[p];
 }
 
