@@ -383,12 +383,14 @@ void emulate_reg_pass(const RegPass& pass, const RegOp* ops, const RegLayout* la
                             uint32_t e0 = 0;
                             for (uint32_t j = 0; j < kRegMaxDiag; ++j) e0 |= ((t >> op.loc[j]) & 1u) << j;
                             const uint32_t off[kRegBits] = {op.nsel, op.selq[0], op.selq[1], op.rcmask};
-                            for (uint32_t u = 0; op.pad && u < kE; ++u) {
+                            for (uint32_t u = 0; op.table && u < kE; ++u) {
                                 uint32_t e = e0;
                                 for (uint32_t i2 = 0; i2 < kRegBits; ++i2)
                                     if ((u >> i2) & 1u) e += off[i2];
                                 cd f;
-                                if (op.nterm) {
+                                if (op.table == kRegTableExpanded) {
+                                    f = mats[op.mat_off + 17 * e0 + u];
+                                } else if (op.nterm) {
                                     const size_t at = dyn_base + op.dyn_table + e;
                                     model.access(dyn_base_slot + at, t, false, "per-tile table read", log,
                                                  tid, pass_index);

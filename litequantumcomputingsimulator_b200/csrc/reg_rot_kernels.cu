@@ -62,13 +62,30 @@ __device__ __forceinline__ void cmul_to(double2& v, double2 f) {
         "}"
         : "+d"(v.x), "+d"(v.y) : "d"(f.x), "d"(f.y));
 }
+// v *= f, w *= g: the products of both before the sums, so that no sum waits for its product.
+__device__ __forceinline__ void cmul_to(double2& v, double2& w, double2 f, double2 g) {
+    asm("{\n\t"
+        ".reg .f64 t, u, p, q;\n\t"
+        "mul.rn.f64 t, %5, %1;\n\t"
+        "mul.rn.f64 u, %5, %0;\n\t"
+        "mul.rn.f64 p, %7, %3;\n\t"
+        "mul.rn.f64 q, %7, %2;\n\t"
+        "neg.f64 t, t;\n\t"
+        "neg.f64 p, p;\n\t"
+        "fma.rn.f64 %0, %4, %0, t;\n\t"
+        "fma.rn.f64 %1, %4, %1, u;\n\t"
+        "fma.rn.f64 %2, %6, %2, p;\n\t"
+        "fma.rn.f64 %3, %6, %3, q;\n\t"
+        "}"
+        : "+d"(v.x), "+d"(v.y), "+d"(w.x), "+d"(w.y)
+        : "d"(f.x), "d"(f.y), "d"(g.x), "d"(g.y));
+}
 
 // a0 += x a1, then a1 += y a0 on register bit TM, both signs toggled by bit 31 of `sign`.  Each
 // FMA overwrites its own addend: computing both new halves from the old ones took a register
 // move for every FMA.
 template <int TM>
-__device__ __forceinline__ void rotation(double2 (&v)[kE], uint32_t mat, uint32_t sign) {
-    const double2 xy = lds2(mat);
+__device__ __forceinline__ void rotation(double2 (&v)[kE], double2 xy, uint32_t sign) {
     const double x = toggle(xy.x, sign), y = toggle(xy.y, sign);
 #pragma unroll
     for (int b = 0; b < kE; ++b) {
@@ -84,28 +101,43 @@ __device__ __forceinline__ void rotation(double2 (&v)[kE], uint32_t mat, uint32_
     }
 }
 
-// Rotations on the register bits of `code`, their (x, y) at `mat` in bit order; bit j of zb: the
-// j-th one's sign.
-__device__ __forceinline__ void rotations(double2 (&v)[kE], uint32_t code, uint32_t mat, uint32_t zb) {
-    if (code & 1u) { rotation<1>(v, mat, zb << 31); mat += 16u; zb >>= 1; }
-    if (code & 2u) { rotation<2>(v, mat, zb << 31); mat += 16u; zb >>= 1; }
-    if (code & 4u) { rotation<4>(v, mat, zb << 31); mat += 16u; zb >>= 1; }
-    if (code & 8u) rotation<8>(v, mat, zb << 31);
+// Rotations on the register bits of `code`, their (x, y) at `mat` in bit order, the first in xy;
+// bit j of zb: the j-th one's sign.  Each (x, y) is loaded before the rotation in front of it
+// (one entry is read past the last: the layouts lie there).
+__device__ __forceinline__ void rotations(double2 (&v)[kE], uint32_t code, uint32_t mat, double2 xy,
+                                          uint32_t zb) {
+    if (code & 1u) { const double2 c = xy; xy = lds2(mat += 16u); rotation<1>(v, c, zb << 31); zb >>= 1; }
+    if (code & 2u) { const double2 c = xy; xy = lds2(mat += 16u); rotation<2>(v, c, zb << 31); zb >>= 1; }
+    if (code & 4u) { const double2 c = xy; xy = lds2(mat += 16u); rotation<4>(v, c, zb << 31); zb >>= 1; }
+    if (code & 8u) rotation<8>(v, xy, zb << 31);
 }
 
-// Diagonal table: amplitude u takes the entry at addr + the strides of u's register bits (zero
-// for bits the table does not use).  One code path for every set of register bits: a switch
-// over them (2^r loads instead of 16) made the allocator spill 600 bytes per thread, and a
-// load of one entry by a whole warp costs 1.2 cycles of the SM, against 2 for the four FMAs it
-// feeds.
-__device__ __forceinline__ void reg_table(double2 (&v)[kE], uint32_t addr, uint32_t s0, uint32_t s1,
-                                          uint32_t s2, uint32_t s3) {
+// Diagonal tables.  One code path for every set of register bits: a switch over them (2^r loads
+// instead of 16) made the allocator spill 600 bytes per thread, and a load of one entry by a
+// whole warp costs 1.2 cycles of the SM, against 2 for the four FMAs it feeds.  Expanded: entry u
+// of the thread's sixteen.
+__device__ __forceinline__ void table_expanded(double2 (&v)[kE], uint32_t addr) {
+    double2 f = lds2(addr), g = lds2(addr + 16u);
 #pragma unroll
-    for (int u = 0; u < kE; ++u) {
-        const double2 f = lds2(addr + ((u & 1) ? s0 : 0u) + ((u & 2) ? s1 : 0u) +
-                               ((u & 4) ? s2 : 0u) + ((u & 8) ? s3 : 0u));
-        cmul_to(v[u], f);
+    for (int u = 0; u < kE; u += 2) {   // the next two entries on their way
+        double2 f1, g1;
+        if (u + 2 < kE) {
+            f1 = lds2(addr + 16u * (u + 2));
+            g1 = lds2(addr + 16u * (u + 3));
+        }
+        cmul_to(v[u], v[u + 1], f, g);
+        f = f1;
+        g = g1;
     }
+}
+// Strided: the entry at addr + the strides of u's register bits (zero for bits the table does
+// not use).
+__device__ __forceinline__ void table_strided(double2 (&v)[kE], uint32_t addr, uint32_t s0, uint32_t s1,
+                                              uint32_t s2, uint32_t s3) {
+#pragma unroll
+    for (int u = 0; u < kE; ++u)
+        cmul_to(v[u], lds2(addr + ((u & 1) ? s0 : 0u) + ((u & 2) ? s1 : 0u) + ((u & 4) ? s2 : 0u) +
+                           ((u & 8) ? s3 : 0u)));
 }
 
 // A pass and its records as a kernel parameter: the record loop then decodes them with
@@ -265,24 +297,31 @@ k_regrot(double2* __restrict__ st, const __grid_constant__ RotPass rp,
         uint32_t cur = 0;
         for (uint32_t o = 0; o < p.n_ops; ++o) {
             // a = {gcmask, mat_off, kind | code | k | rcmask}, b = {tcmask | loc[0..1],
-            // loc[2..5], nsel | selq[0..1] | nterm, dyn_off | pad}
+            // loc[2..5], nsel | selq[0..1] | nterm, dyn_off | table}
             const uint4* rec = reinterpret_cast<const uint4*>(&rp.ops[o]);
             const uint4 a = rec[0], b = rec[1];
             const uint32_t kind = a.w & 0xffu, code = (a.w >> 8) & 0xffu;
             const uint32_t mat = smat_addr + 16u * a.z;
             if (kind == kRegStage) {
-                if (b.w & 0x10000u) {   // the table
+                const uint32_t form = (b.w >> 16) & 0xffu;
+                const uint32_t at = smat_addr + 16u * (b.w & 0xffffu);
+                const double2 xy = lds2(at);   // the first rotation's, if there is one
+                if (form) {   // the table
                     const uint32_t t = threadIdx.x;
-                    const uint32_t e = ((t >> ((b.x >> 16) & 31u)) & 1u) | ((t >> ((b.x >> 24) & 31u)) & 1u) << 1 |
-                                       ((t >> (b.y & 31u)) & 1u) << 2 | ((t >> ((b.y >> 8) & 31u)) & 1u) << 3 |
-                                       ((t >> ((b.y >> 16) & 31u)) & 1u) << 4 |
-                                       ((t >> ((b.y >> 24) & 31u)) & 1u) << 5;
-                    const uint32_t tab = (b.z >> 24) ? sdyn_addr + 16u * (dyn_base + (a.x & 0xffffu)) : mat;
-                    reg_table(v, tab + 16u * e, (b.z & 0xffu) << 4, (b.z >> 4) & 0xff0u,
-                              (b.z >> 12) & 0xff0u, (a.w >> 20) & 0xff0u);
+                    uint32_t e = ((t >> ((b.x >> 16) & 31u)) & 1u) | ((t >> ((b.x >> 24) & 31u)) & 1u) << 1 |
+                                 ((t >> (b.y & 31u)) & 1u) << 2;
+                    if (form == kRegTableExpanded) {
+                        table_expanded(v, mat + 272u * e);
+                    } else {
+                        e |= ((t >> ((b.y >> 8) & 31u)) & 1u) << 3 | ((t >> ((b.y >> 16) & 31u)) & 1u) << 4 |
+                             ((t >> ((b.y >> 24) & 31u)) & 1u) << 5;
+                        const uint32_t tab = (b.z >> 24) ? sdyn_addr + 16u * (dyn_base + (a.x & 0xffffu)) : mat;
+                        table_strided(v, tab + 16u * e, (b.z & 0xffu) << 4, (b.z >> 4) & 0xff0u,
+                                      (b.z >> 12) & 0xff0u, (a.w >> 20) & 0xff0u);
+                    }
                 }
                 if (code) {
-                    const uint32_t at = smat_addr + 16u * (b.w & 0xffffu), sg = b.x & 0xffffu;
+                    const uint32_t sg = b.x & 0xffffu;
                     uint32_t zb = static_cast<uint32_t>(signs >> sg);
                     if (sg > kRegSignBits) {   // lane j: the sign of the j-th rotation
                         const uint32_t nr = static_cast<uint32_t>(__popc(code));
@@ -290,7 +329,7 @@ k_regrot(double2* __restrict__ st, const __grid_constant__ RotPass rp,
                         if (lane < nr) odd = (__popcll(base & mask_at(at + 16u * (nr + lane))) & 1) != 0;
                         zb = __ballot_sync(0xffffffffu, odd);
                     }
-                    rotations(v, code, at, zb);
+                    rotations(v, code, at, xy, zb);
                 }
                 continue;
             }
@@ -415,7 +454,9 @@ void launch_variant(const LaunchCtx& ctx, double2* st, uint32_t batch, const Reg
 template <int M, int MINB>
 void launch_size(const LaunchCtx& ctx, double2* st, uint32_t batch, const RegPass& p, size_t smem,
                  const RegOp* ops, const RegLayout* d_layouts, const double2* d_mats) {
-    if (!p.pauli_ops && p.fma_dense)
+    if (!p.pauli_ops && !p.fma_dense)
+        launch_variant<M, MINB, false, false>(ctx, st, batch, p, smem, ops, d_layouts, d_mats);
+    else if (!p.pauli_ops)
         launch_variant<M, MINB, true, false>(ctx, st, batch, p, smem, ops, d_layouts, d_mats);
     else if (!p.fma_dense)
         launch_variant<M, MINB, false, true>(ctx, st, batch, p, smem, ops, d_layouts, d_mats);

@@ -111,10 +111,13 @@ constexpr uint32_t kRegPauliMaxFlips = 9;       // X/Y qubits of a Pauli rotatio
 // its matrices: (cos, 0), y, then the mask as two exact 32-bit halves).
 //
 // Passes in rotation form (RegPass::rot, reg_rot_kernels.cu) have four more:
-// kRegStage: an optional diagonal table, then rotations.  The table (pad = 1) covers k tile
-// bits; entry bit j is thread bit loc[j] (31: none), register bit i adds the entry offset nsel,
-// selq[0], selq[1], rcmask (i = 0..3; 0 if the table does not use it); with nterm gated terms it
-// is built per tile (at dyn_table among the per-tile tables) like kRegDiagDyn's.  A rotation is
+// kRegStage: an optional diagonal table, then rotations.  The table covers k tile bits.
+// kRegTableStrided: entry bit j is thread bit loc[j] (31: none), register bit i adds the entry
+// offset nsel, selq[0], selq[1], rcmask (i = 0..3; 0 if the table does not use it); with nterm
+// gated terms it is built per tile (at dyn_table among the per-tile tables) like kRegDiagDyn's.
+// kRegTableExpanded: at most kRegTableThreadBits thread bits loc[0..2]; sixteen entries by register
+// index for each of their values, which lie 17 entries apart (so that lanes that differ in them
+// read different banks).  A rotation is
 // a0 += x a1, then a1 += y a0 with real x, y, on each register bit of `code`: what is left of a
 // one-qubit gate once its diagonal factors have moved into the neighbouring tables; their (x, y)
 // are at dyn_off among the matrices, bits ascending.  tcmask: the index of their signs (of x and
@@ -127,6 +130,8 @@ constexpr uint32_t kRegPauliMaxFlips = 9;       // X/Y qubits of a Pauli rotatio
 // per mask, those that negate it where they are all 1.
 enum : uint8_t { kRegDense = 0, kRegDiag = 1, kRegPhase = 2, kRegSwapX = 3, kRegRemap = 4,
                  kRegDiagDyn = 5, kRegMma = 6, kRegPauli = 7, kRegStage = 8, kRegSign = 9 };
+enum : uint8_t { kRegTableExpanded = 1, kRegTableStrided = 2 };
+constexpr uint32_t kRegTableThreadBits = 3;
 constexpr uint32_t kRegSignBits = 60;   // sign bits of a tile (64-bit word, the top ones 0)
 
 struct RegLayout {
@@ -154,8 +159,8 @@ struct alignas(16) RegOp {
     uint8_t selq[kRegMaxSelect];   // one of 2^nsel consecutive matrices
     uint8_t nterm;            // per-tile diagonal: gated phase terms; rotation, sign: see above
     uint16_t dyn_off;         // per-tile diagonal: first entry in the per-tile tables
-    uint8_t pad;              // stage: has a table
-    uint8_t pad2;
+    uint8_t table;            // stage: kRegTable...
+    uint8_t pad;
 };
 
 struct RegPass {

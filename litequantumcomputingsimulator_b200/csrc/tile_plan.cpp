@@ -1625,13 +1625,13 @@ class DiagonalPool {
     }
     // Emits one table that takes waiting operations on bits of `touch`.
     void flush(uint32_t touch, Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
-        emit(group(touch), e, ly, S, m);
+        emit(group(touch, S), e, ly, S, m);
     }
     void flush_all(Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
         while (!items_.empty()) {
             uint32_t touch = 0;
             for (const Item& it : items_) touch |= it.bits;
-            emit(touch ? group(touch) : 0u, e, ly, S, m);
+            emit(touch ? group(touch, S) : 0u, e, ly, S, m);
         }
     }
 
@@ -1660,22 +1660,32 @@ class DiagonalPool {
     }
 
     // Tile bits of the next table: whole components of joined bits while they fit, first those
-    // with a bit of `touch`; if the first is too wide, as much of it as fits.
-    uint32_t group(uint32_t touch) const {
-        const int most = static_cast<int>(kRegMaxDiag);
-        uint32_t u = 0;
-        for (int round = 0; round < 2; ++round)
-            for (const Item& it : items_) {
-                if ((it.bits & u) || (round == 0 && !(it.bits & touch))) continue;
-                const uint32_t c = closure(it.bits);
-                if (!(c & u) && width(u | c) <= most) u |= c;
-            }
-        if (u & touch) return u;
-        u = 0;
-        for (int round = 0; round < 2; ++round)   // what touches, then what is joined to that
-            for (const Item& it : items_)
-                if ((it.bits & (round ? u : touch)) && width(u | it.bits) <= most) u |= it.bits;
-        return u;
+    // with a bit of `touch`; if the first is too wide, as much of it as fits.  Fitting: at most
+    // three thread bits beside the register bits S (an expanded table); with gated phases about,
+    // or where nothing fits so, six bits (a strided one, which a tile may build).
+    uint32_t group(uint32_t touch, uint32_t S) const {
+        bool gated = false;
+        for (const Item& it : items_) gated |= it.op->kind == kTilePhase && it.op->gcmask != 0;
+        for (int strided = gated ? 1 : 0; strided < 2; ++strided) {
+            auto fits = [&](uint32_t bits) {
+                return strided ? width(bits) <= static_cast<int>(kRegMaxDiag)
+                               : width(bits & ~S) <= static_cast<int>(kRegTableThreadBits);
+            };
+            uint32_t u = 0;
+            for (int round = 0; round < 2; ++round)
+                for (const Item& it : items_) {
+                    if ((it.bits & u) || (round == 0 && !(it.bits & touch))) continue;
+                    const uint32_t c = closure(it.bits);
+                    if (!(c & u) && fits(u | c)) u |= c;
+                }
+            if (u & touch) return u;
+            u = 0;
+            for (int round = 0; round < 2; ++round)   // what touches, then what is joined to that
+                for (const Item& it : items_)
+                    if ((it.bits & (round ? u : touch)) && fits(u | it.bits)) u |= it.bits;
+            if (u & touch) return u;
+        }
+        logic("register tile lowering: a diagonal too wide for a table");
     }
 
     // One table over the tile bits `u`: the product of every waiting operation within them,
@@ -1684,6 +1694,7 @@ class DiagonalPool {
     void emit(uint32_t u, Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
         RegOp r{};
         std::vector<uint32_t> bits;
+        const bool narrow_enough = width(u & ~S) <= static_cast<int>(kRegTableThreadBits);
         for (uint8_t& l : r.loc) l = 31;
         for (uint32_t i = 0; i < m - kRegBits; ++i)
             if ((u >> ly.tpos[i]) & 1) {
@@ -1729,7 +1740,7 @@ class DiagonalPool {
         }
         if (!members.empty() || !gated.empty()) {
             const cl one{1, 0};
-            cl bit[kRegMaxDiag][2];
+            cl bit[kRegBits + kRegMaxDiag][2];
             for (uint32_t j = 0; j < k; ++j) bit[j][0] = bit[j][1] = one;
             for (const LocalOp* o : members) {   // one-bit factors first: a product per bit
                 if (o->kind == kTileDiag && o->lt.size() == 1) {
@@ -1764,11 +1775,24 @@ class DiagonalPool {
             }
             e.close();
             r.kind = kRegStage;
-            r.pad = 1;
+            r.table = gated.empty() && narrow_enough ? kRegTableExpanded : kRegTableStrided;
             r.nterm = static_cast<uint8_t>(gated.size());
             r.mat_off = static_cast<uint32_t>(e.mats.size());
             const uint32_t flip = entry_mask(u & e.flipped);
-            for (uint32_t x = 0; x < size; ++x) e.mats.push_back(narrow(table[x ^ flip]));
+            if (r.table == kRegTableExpanded) {
+                const uint32_t threads = 1u << width(u & ~S);
+                for (uint32_t t = 0; t < threads; ++t) {
+                    for (uint32_t v = 0; v < (1u << kRegBits); ++v) {
+                        uint32_t x = t;
+                        for (uint32_t i = 0; i < kRegBits; ++i)
+                            if ((v >> i) & 1) x += *reg_offset[i];
+                        e.mats.push_back(narrow(table[x ^ flip]));
+                    }
+                    e.mats.emplace_back(0.0, 0.0);
+                }
+            } else {
+                for (uint32_t x = 0; x < size; ++x) e.mats.push_back(narrow(table[x ^ flip]));
+            }
             for (const LocalOp* o : gated) {
                 const uint32_t em = entry_mask(o->lmask);
                 append_term(o->m[0], o->gcmask, em, em & ~flip, e.mats);
