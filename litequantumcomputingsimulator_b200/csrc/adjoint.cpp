@@ -431,14 +431,23 @@ struct AdjointPlan {
         }
     }
 
-    // Passes of rotations for both sweeps: register passes (adj_pass.cuh) from 9 qubits, forward
-    // tiles of 2^min(n, 12) amplitudes (16 per thread), backward 2^min(n, 11) (8 of psi and 8 of
-    // lambda); below, where a tile has fewer amplitudes than a warp's registers, rotation tile
-    // passes in shared memory.  LQCS_ADJ_TILES=0 keeps one launch per step.
+    // Passes of rotations for both sweeps: register passes (adj_pass.cuh) from 9 qubits, 16
+    // amplitudes per thread forward, 8 of psi and 8 of lambda backward; below, where a tile has
+    // fewer amplitudes than a warp's registers, rotation tile passes in shared memory.  A CTA
+    // loads, computes and stores its tile one after the other, so what overlaps is the work of
+    // different CTAs of an SM: smaller tiles (more CTAs of the same 512 threads, each at another
+    // stage) run faster although they take more passes.  Measured, forward 2^12 / backward 2^11
+    // against 2^11 and the backward sizes below: 16 qubits, 200 rotations, 256 sets 17.0 -> 15.5
+    // ms (2^10 backward 15.9); 13..15 qubits 2^10 and 2^9 backward tie (64 to 256 sets: 5 % under
+    // 2^11, 20 rotations of 15 qubits: 1.02, 0.99, 1.10 ms for 2^11, 2^10, 2^9); at 12 qubits and
+    // below the extra passes cost more (0.25 against 0.26 ms), and above 20 the sizes tie while
+    // 2^9 needs four times the gradient partials.
+    // LQCS_ADJ_TILES=0 keeps one launch per step.
     void plan_tiles() {
         if (env_or("LQCS_ADJ_TILES", 1) == 0) return;
-        const uint32_t mf = std::min<uint32_t>(n, static_cast<uint32_t>(env_or("LQCS_ADJ_TILE_F", 12)));
-        const uint32_t mb = std::min<uint32_t>(n, static_cast<uint32_t>(env_or("LQCS_ADJ_TILE_B", 11)));
+        const int back_bits = n > 20 ? 11 : n >= 16 ? 9 : n >= 13 ? 10 : 11;
+        const uint32_t mf = std::min<uint32_t>(n, static_cast<uint32_t>(env_or("LQCS_ADJ_TILE_F", 11)));
+        const uint32_t mb = std::min<uint32_t>(n, static_cast<uint32_t>(env_or("LQCS_ADJ_TILE_B", back_bits)));
         if (mf < 5 || mb < 5 || mf > kRotMaxBits || mb > kRotMaxBits) return;
         const uint32_t L = 3;
         std::vector<RotTileOp> ops;

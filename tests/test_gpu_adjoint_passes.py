@@ -67,6 +67,21 @@ def test_passes_equal_one_launch_per_step(monkeypatch, n, sets, ccx):
     assert np.array_equal(again[0], energies) and np.array_equal(again[1], grads)
 
 
+@pytest.mark.parametrize("n", [20, 21])   # the backward tiles' size changes between them
+def test_tile_sizes_of_large_registers(monkeypatch, n):
+    pc = ansatz(n, 14, 200 + n)
+    ham = W.random_hamiltonian(n, 6, seed=n)
+    scale = sum(abs(c) for c, _ in ham)
+    params = W.random_parameter_sets(pc.num_parameters(), 2, seed=n + 1)
+    energies, grads = A.adjoint_gradient(ham, pc, params)
+    A.release_caches()
+    monkeypatch.setenv("LQCS_ADJ_TILES", "0")
+    want_e, want_g = A.adjoint_gradient(ham, pc, params)
+    A.release_caches()
+    assert np.max(np.abs(energies - want_e)) < 1e-12 * scale
+    assert np.max(np.abs(grads - want_g)) < 2e-12 * scale
+
+
 def test_gradient_against_central_differences():
     pc = ansatz(10, 30, 5)
     ham = W.random_hamiltonian(10, 20, seed=6)
