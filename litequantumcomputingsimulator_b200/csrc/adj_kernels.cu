@@ -343,12 +343,15 @@ __device__ __forceinline__ double term_factor(bool pairs, uint32_t n_y) {
 }
 
 // Persistent CTAs over the tiles; each thread keeps a sum per term (in shared memory), added up
-// tile after tile, and the block's sums go out once.  HBM-bound: 16 bytes per amplitude for up
-// to nine independent x masks, where a launch per x mask read the state for each.
-__global__ void __launch_bounds__(256, 2) k_expect_pass(const double2* __restrict__ s,
-                                                        uint32_t n_tiles,
-                                                        const __grid_constant__ AdjPass p,
-                                                        double* __restrict__ partials) {
+// tile after tile, and the block's sums go out once.  A read of the state (16 bytes per amplitude)
+// serves up to eight independent x masks, where a launch per x mask read it for each.  A CTA loads
+// a tile and sums it one after the other, so the CTAs of an SM overlap with each other only: four
+// on tiles of 2^11 beat two on 2^12 (nine masks a read) and eight on 2^10.  100 terms on 24 qubits:
+// 7.09 ms with a launch per mask, 1.25 with 2^12, 0.95 with 2^11, 1.00 with 2^10, 1.06 with 2^9;
+// 150 terms on 26 qubits 6.6 (2^12), 4.8 (2^11); 40 terms on 15 qubits 0.092 both.
+__global__ void __launch_bounds__(kExpectThreads, kExpectCtas)
+k_expect_pass(const double2* __restrict__ s, uint32_t n_tiles, const __grid_constant__ AdjPass p,
+              double* __restrict__ partials) {
     constexpr int M = kExpectTileBits, TB = M - 4, E = 16;
     constexpr uint32_t T = 1u << TB;
     extern __shared__ __align__(16) double2 tile[];
@@ -478,7 +481,7 @@ void bwd(const LaunchCtx& ctx, double2* psi, double2* lam, uint32_t n, uint32_t 
 }  // namespace
 
 uint32_t expect_blocks(const LaunchCtx& ctx, uint32_t n) {
-    return std::min<uint32_t>(1u << (n - kExpectTileBits), static_cast<uint32_t>(ctx.num_sms) * 2);
+    return std::min<uint32_t>(1u << (n - kExpectTileBits), static_cast<uint32_t>(ctx.num_sms) * kExpectCtas);
 }
 
 void launch_expect_pass(const LaunchCtx& ctx, const double2* st, uint32_t n, const AdjPass& p,
@@ -488,7 +491,7 @@ void launch_expect_pass(const LaunchCtx& ctx, const double2* st, uint32_t n, con
     const size_t smem = (sizeof(double2) << kExpectTileBits) + sizeof(double) * p.n_rots * (1u << (kExpectTileBits - 4));
     cuda_check_launch_attr(cudaFuncSetAttribute(k_expect_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 static_cast<int>(smem)));
-    k_expect_pass<<<expect_blocks(ctx, n), 256, smem, ctx.stream>>>(st, 1u << (n - kExpectTileBits), p, d_partials);
+    k_expect_pass<<<expect_blocks(ctx, n), kExpectThreads, smem, ctx.stream>>>(st, 1u << (n - kExpectTileBits), p, d_partials);
     check_launch("expectation pass");
 }
 

@@ -58,7 +58,8 @@ std::vector<AdjPass> plan_adjoint_passes(const std::vector<AdjRotation>& rots, u
 
 // Pauli expectations <psi|P|psi> of terms i^n_y X^x Z^zy on the same tiles: a pass reads the state
 // once for every term whose x lies in its tiles' subspace.  param: the term's place in d_out.
-constexpr uint32_t kExpectTileBits = 12, kExpectTerms = 20;   // per pass
+constexpr uint32_t kExpectTileBits = 11, kExpectTerms = 20;   // per pass
+constexpr uint32_t kExpectThreads = 1u << (kExpectTileBits - 4), kExpectCtas = 512 / kExpectThreads;
 constexpr uint32_t kExpectSmall = 14;                         // to here: a block per term
 uint32_t expect_blocks(const LaunchCtx& ctx, uint32_t n);      // partials per term, n > kExpectSmall
 void launch_expect_pass(const LaunchCtx& ctx, const double2* st, uint32_t n, const AdjPass& p,
