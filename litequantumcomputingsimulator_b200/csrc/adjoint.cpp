@@ -137,8 +137,8 @@ void HamiltonianDev::upload(const Hamiltonian& h, uint32_t n) {
 namespace {
 
 // Resident sets per launch batch: as many as fit (two states per set), at most 256.  With
-// the rotation tile passes a launch is compute-heavy and larger batches amortise it better
-// (16 qubits: 7960 gradients/s with 256 sets, 7570 with 32).  One launch per step (fixed
+// passes a launch is compute-heavy and larger batches amortise it better (16 qubits, passes in
+// shared memory: 7960 gradients/s with 256 sets, 7570 with 32).  One launch per step (fixed
 // gates, LQCS_ADJ_TILES=0) streams every state per step, and there a batch that stays in L2
 // is faster (32 sets: 4230 against 3210) — max_resident picks that size.
 uint32_t default_resident(uint32_t n, uint64_t batch) {
