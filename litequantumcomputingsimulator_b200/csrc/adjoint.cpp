@@ -363,6 +363,7 @@ struct AdjointPlan {
     AdjointPlan(const AdjointPlan&) = delete;
     AdjointPlan& operator=(const AdjointPlan&) = delete;
     ~AdjointPlan() {
+        if (stream) StreamDrain{stream};   // a call that failed leaves work behind
         for (auto& g : graphs) cudaGraphExecDestroy(g.second.first);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -868,6 +869,7 @@ struct MultiPlan {
     MultiPlan(const MultiPlan&) = delete;
     MultiPlan& operator=(const MultiPlan&) = delete;
     ~MultiPlan() {
+        if (origin) StreamDrain{origin};
         if (exec) cudaGraphExecDestroy(exec);
         for (cudaEvent_t e : joins) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);

@@ -321,7 +321,7 @@ int lqcs_state_probabilities(const lqcs_state* st, double* host_out) {
     return guarded([&] {
         need(st, "state");
         need(host_out, "host_out");
-        lqcs_b200::DeviceBuffer p;
+        lqcs_b200::DeviceBuffer p(st->stream);
         p.ensure(sizeof(double) * st->len());
         lqcs_b200::launch_probabilities(st->ctx, st->d(), st->n, p.as<double>());
         lqcs_b200::cuda_check(cudaMemcpyAsync(host_out, p.ptr, sizeof(double) * st->len(),

@@ -94,7 +94,7 @@ std::unique_ptr<lqcs_state> dm_evolve(uint32_t n, const std::vector<GateDesc>& g
 }
 
 void dm_probabilities(lqcs_state& rho, uint32_t n, double* host) {
-    DeviceBuffer p;
+    DeviceBuffer p(rho.stream);
     p.ensure(sizeof(double) << n);
     launch_dm_diagonal(rho.ctx, rho.d(), n, p.as<double>());
     cuda_check(cudaMemcpyAsync(host, p.ptr, sizeof(double) << n, cudaMemcpyDeviceToHost,

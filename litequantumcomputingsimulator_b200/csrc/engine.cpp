@@ -2,6 +2,7 @@
 #include "engine.hpp"
 
 #include "adj_pass.cuh"
+#include "block_pool.hpp"
 #include "costmodel.hpp"
 
 #include <algorithm>
@@ -28,85 +29,55 @@ void cuda_check(cudaError_t e, const char* what) {
 
 namespace {
 
-constexpr size_t kBlockMax = size_t{32} << 20, kIdleMax = size_t{256} << 20;
-// Blocks of up to 1 MiB are cut from slabs of 8 MiB: a plan or a program needs a dozen of them.
-constexpr size_t kSlabBlockMax = size_t{1} << 20, kSlab = size_t{8} << 20;
-
-struct BlockPool {
-    struct Slab {
-        char* base;
-        size_t used;   // bytes cut so far
-        size_t live;   // blocks in use
+// The pool's CUDA calls.  None leaves its error in the thread's last-error slot, which the next
+// launch check reads.
+struct CudaBlocks {
+    struct Current {   // the calling thread's device, put back at the end
+        int cur = 0;
+        explicit Current(int device) {
+            if (cudaGetDevice(&cur) != cudaSuccess) cudaGetLastError();
+            if (cur != device && cudaSetDevice(device) != cudaSuccess) cudaGetLastError();
+        }
+        ~Current() { cudaSetDevice(cur); }
     };
-    std::mutex mu;
-    std::map<std::pair<int, size_t>, std::vector<void*>> idle;
-    std::map<int, size_t> idle_bytes;
-    std::map<int, std::vector<Slab>> slabs;
-
-    Slab* slab_of(int device, void* p) {
-        for (Slab& s : slabs[device])
-            if (p >= s.base && p < s.base + kSlab) return &s;
-        return nullptr;
+    static void* allocate(int device, size_t bytes) {
+        Current on(device);
+        void* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        cuda_check(e, "cudaMalloc");
+        return p;
     }
-    // Idle blocks and slabs without a block in use, taken out of the pool (to be freed).
-    std::vector<std::pair<int, void*>> take_idle() {
-        std::vector<std::pair<int, void*>> drop;
-        for (auto& [key, ptrs] : idle) {
-            std::vector<void*> keep;
-            for (void* p : ptrs) {
-                const Slab* s = key.second <= kSlabBlockMax ? slab_of(key.first, p) : nullptr;
-                if (s && s->live > 0) {
-                    keep.push_back(p);
-                    continue;
-                }
-                idle_bytes[key.first] -= key.second;
-                if (!s) drop.emplace_back(key.first, p);
-            }
-            ptrs.swap(keep);
-        }
-        for (auto& [dev, list] : slabs) {
-            std::vector<Slab> keep;
-            for (const Slab& s : list) {
-                if (s.live > 0) keep.push_back(s);
-                else drop.emplace_back(dev, s.base);
-            }
-            list.swap(keep);
-        }
-        return drop;
+    static bool free(int device, void* p) {
+        Current on(device);
+        if (cudaFree(p) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
+    // Waits for the stream's work.  False where that is not possible: the stream (or one that the
+    // default stream would wait for) is being captured, or the device has failed.
+    static bool wait(int device, cudaStream_t stream) {
+        Current on(device);
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &c) == cudaSuccess &&
+            (c != cudaStreamCaptureStatusNone || cudaStreamSynchronize(stream) == cudaSuccess))
+            return c == cudaStreamCaptureStatusNone;
+        cudaGetLastError();
+        return false;
     }
 };
-BlockPool& blocks() {   // never destroyed: buffers may be freed during process exit
-    static auto* p = new BlockPool;
+
+BlockPool<CudaBlocks>& blocks() {   // never destroyed: buffers may be freed during process exit
+    static auto* p = new BlockPool<CudaBlocks>;
     return *p;
-}
-
-void free_all(const std::vector<std::pair<int, void*>>& drop) {
-    int cur = 0;
-    cudaGetDevice(&cur);
-    for (const auto& [dev, p] : drop) {
-        cudaSetDevice(dev);
-        cudaFree(p);
-    }
-    if (!drop.empty()) cudaSetDevice(cur);
-}
-
-// Capacity of a block for b bytes: the next of 4, 5, 6, 7 times a power of two, 512 at least.
-size_t block_size(size_t b) {
-    size_t step = 128;
-    while (step * 8 < b) step <<= 1;
-    return std::max<size_t>(512, (b + step - 1) / step * step);
 }
 
 }  // namespace
 
-void clear_buffer_pool() {
-    std::vector<std::pair<int, void*>> drop;
-    {
-        std::lock_guard<std::mutex> lk(blocks().mu);
-        drop = blocks().take_idle();
-    }
-    free_all(drop);
-}
+void clear_buffer_pool() { blocks().clear(); }
 
 void DeviceBuffer::release() {
     if (!ptr) return;
@@ -114,81 +85,22 @@ void DeviceBuffer::release() {
     const size_t b = bytes;
     ptr = nullptr;
     bytes = 0;
-    if (b > kBlockMax) {
-        cudaFree(p);
-        return;
-    }
-    int cur = 0;
-    const bool known = cudaGetDevice(&cur) == cudaSuccess;
-    if (known && cur != device) cudaSetDevice(device);
-    const bool done = known && cudaDeviceSynchronize() == cudaSuccess;
-    if (known && cur != device) cudaSetDevice(cur);
-    std::vector<std::pair<int, void*>> drop;
-    {
-        std::lock_guard<std::mutex> lk(blocks().mu);
-        BlockPool::Slab* s = b <= kSlabBlockMax ? blocks().slab_of(device, p) : nullptr;
-        if (!done) {
-            // the device did not come to rest (a failed context, process exit): a block of its
-            // own goes back to the driver, one cut from a slab is never handed out again
-            if (!s) drop.emplace_back(device, p);
-        } else {
-            if (s) --s->live;
-            size_t& total = blocks().idle_bytes[device];
-            blocks().idle[{device, b}].push_back(p);
-            total += b;
-            if (total > kIdleMax) drop = blocks().take_idle();
-        }
-    }
-    free_all(drop);
+    if (b > kBlockMax) blocks().discard(device, p);
+    else blocks().give(device, p, b, CudaBlocks::wait(device, stream));
 }
 
 void DeviceBuffer::ensure(size_t b) {
     if (b <= bytes) return;
     release();
     cuda_check(cudaGetDevice(&device), "cudaGetDevice");
-    const size_t want = b <= kBlockMax ? block_size(b) : b;
-    const bool slab = want <= kSlabBlockMax;
-    // an idle block, or one cut from a slab
-    auto take = [&](bool cut) -> void* {
-        BlockPool& pool = blocks();
-        const auto it = pool.idle.find({device, want});
-        if (it != pool.idle.end() && !it->second.empty()) {
-            void* p = it->second.back();
-            it->second.pop_back();
-            pool.idle_bytes[device] -= want;
-            if (BlockPool::Slab* s = slab ? pool.slab_of(device, p) : nullptr) ++s->live;
-            return p;
-        }
-        if (!cut) return nullptr;
-        for (BlockPool::Slab& s : pool.slabs[device])
-            if (s.used + want <= kSlab) {
-                void* p = s.base + s.used;
-                s.used += want;
-                ++s.live;
-                return p;
-            }
-        return nullptr;
-    };
-    if (want <= kBlockMax) {
-        std::lock_guard<std::mutex> lk(blocks().mu);
-        ptr = take(slab);
+    if (b <= kBlockMax) {
+        ptr = blocks().take(device, b);
+    } else if (!(ptr = CudaBlocks::allocate(device, b))) {   // once more without the idle blocks
+        clear_buffer_pool();
+        ptr = CudaBlocks::allocate(device, b);
     }
-    if (!ptr) {
-        void* fresh = nullptr;
-        cudaError_t e = cudaMalloc(&fresh, slab ? kSlab : want);
-        if (e == cudaErrorMemoryAllocation) {   // once more without the idle blocks
-            cudaGetLastError();
-            clear_buffer_pool();
-            e = cudaMalloc(&fresh, slab ? kSlab : want);
-        }
-        cuda_check(e, "cudaMalloc");
-        if (slab) {
-            std::lock_guard<std::mutex> lk(blocks().mu);
-            blocks().slabs[device].push_back({static_cast<char*>(fresh), want, 1});
-        }
-        ptr = fresh;
-    }
-    bytes = want;
+    if (!ptr) cuda_check(cudaErrorMemoryAllocation, "cudaMalloc");
+    bytes = b <= kBlockMax ? block_size(b) : b;
 }
 
 int device_sm_count() {
@@ -604,6 +516,7 @@ static std::vector<double> time_candidates(const std::vector<GateDesc>& gates, u
     auto st = new_state(n, 1, s);
     for (const TuneCandidate& c : cands) {
         Program p = compile_candidate(gates, n, c, s);
+        const StreamDrain drain{s};
         p.launch(st->ctx, st->d(), n, 1);   // untimed: first-launch set-up
         cuda_check(cudaEventRecord(guard.a, s), "cudaEventRecord");
         p.launch(st->ctx, st->d(), n, 1);
@@ -826,20 +739,14 @@ void clear_state_pool() {
         std::lock_guard<std::mutex> lk(pool_mu());
         drop.swap(pool());
     }
-    int cur = 0;
-    cudaGetDevice(&cur);
-    for (const PooledBuffer& b : drop) {
-        cudaSetDevice(b.device);
-        cudaFree(b.ptr);
-    }
-    cudaSetDevice(cur);
+    for (const PooledBuffer& b : drop) blocks().discard(b.device, b.ptr);
 }
 
 void pool_return(lqcs_state& st) {
     // (smaller ones are the block pool's)
     if (!st.amps.ptr || st.amps.bytes <= kBlockMax || st.amps.bytes > kPoolMaxBytes) return;
     // the buffer is reused only after this state's work on it has finished
-    if (cudaStreamSynchronize(st.stream) != cudaSuccess) return;
+    if (!CudaBlocks::wait(st.device, st.stream)) return;
     void* evict = nullptr;
     int evict_dev = 0;
     {
@@ -853,13 +760,7 @@ void pool_return(lqcs_state& st) {
     }
     st.amps.ptr = nullptr;
     st.amps.bytes = 0;
-    if (evict) {
-        int cur = 0;
-        cudaGetDevice(&cur);
-        cudaSetDevice(evict_dev);
-        cudaFree(evict);
-        cudaSetDevice(cur);
-    }
+    if (evict) blocks().discard(evict_dev, evict);
 }
 
 std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t stream) {
@@ -883,7 +784,7 @@ std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t s
     cuda_check(cudaGetDevice(&st->device), "cudaGetDevice");
     st->n = n;
     st->batch = batch;
-    st->stream = stream;
+    st->stream = st->amps.stream = st->scratch.stream = st->sample_scratch.stream = stream;
     st->ctx = make_ctx(stream);
     const size_t bytes = sizeof(double2) * st->len() * batch;
     if (void* p = pool_take(st->device, bytes)) {

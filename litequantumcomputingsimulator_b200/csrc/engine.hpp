@@ -17,18 +17,22 @@ namespace lqcs_b200 {
 void cuda_check(cudaError_t e, const char* what);
 
 // Owning device allocation.  Blocks of up to 32 MiB come from and go back to a pool that all
-// buffers of a device share (at most 256 MiB lie idle in it; lqcs_release_caches and a failed
-// allocation empty it): cudaMalloc and cudaFree cost 0.1 to 10 ms a call on a shared host, more
-// than the kernels of a 20-qubit run.  Like cudaFree, release() first waits for the device, so
-// a block is idle when it is handed out again, whatever streams used it.
+// buffers of a device share (block_pool.hpp): cudaMalloc and cudaFree cost 0.1 to 10 ms a call on a
+// shared host, more than the kernels of a 20-qubit run.  At most 256 MiB lie idle in it, besides
+// those in 8 MiB slabs with a block in use; lqcs_release_caches and a failed allocation empty it.
+// release() waits for `stream`, so a block is idle when it is handed out again: work on other
+// streams must have finished by then.  (Not for the device, as cudaFree does: that would wait
+// for other threads' work, and is an error while any thread captures a graph.)
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
-    DeviceBuffer() = default;
+    cudaStream_t stream = nullptr;
+    explicit DeviceBuffer(cudaStream_t s = nullptr) : stream(s) {}
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-    DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes), device(o.device) {
+    DeviceBuffer(DeviceBuffer&& o) noexcept
+        : ptr(o.ptr), bytes(o.bytes), device(o.device), stream(o.stream) {
         o.ptr = nullptr;
         o.bytes = 0;
     }
@@ -38,6 +42,7 @@ struct DeviceBuffer {
             ptr = o.ptr;
             bytes = o.bytes;
             device = o.device;
+            stream = o.stream;
             o.ptr = nullptr;
             o.bytes = 0;
         }
@@ -47,6 +52,15 @@ struct DeviceBuffer {
     void release();
     void ensure(size_t b);
     template <class T> T* as() const { return static_cast<T*>(ptr); }
+};
+
+// Waits for a stream's work at the end of a scope, whichever way it ends.  Declared after what
+// that work uses.
+struct StreamDrain {
+    cudaStream_t stream;
+    ~StreamDrain() {
+        if (cudaStreamSynchronize(stream) != cudaSuccess) cudaGetLastError();
+    }
 };
 
 int device_sm_count();

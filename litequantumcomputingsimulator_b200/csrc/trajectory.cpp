@@ -163,7 +163,7 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
                   u_perm.begin() + p * f.K);
     std::vector<uint64_t> regs_perm(f.shots);
 
-    DeviceBuffer d_u, part, mats, flag, scale, dregs;
+    DeviceBuffer d_u(cs), part(cs), mats(cs), flag(cs), scale(cs), dregs(cs);
     d_u.ensure(sizeof(double) * std::max<size_t>(1, u_perm.size()));
     if (!u_perm.empty())
         cuda_check(cudaMemcpy(d_u.ptr, u_perm.data(), sizeof(double) * u_perm.size(),
@@ -186,7 +186,7 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
             --tail;
         }
     }
-    DeviceBuffer d_vals;
+    DeviceBuffer d_vals(cs);
     d_vals.ensure(sizeof(uint64_t) * R);
 
     // The host lowers a batch while the device still runs the one before: what the device reads
@@ -197,6 +197,7 @@ void run_fused(const FusedRun& f, uint64_t* regs) {
     };
     std::vector<Held> held;
     size_t held_bytes = 0;
+    const StreamDrain drain{cs};
     for (uint64_t first = 0; first < f.shots;) {   // first: batch start position in `order`
         const uint32_t nb = static_cast<uint32_t>(
             first < n_clean ? std::min<uint64_t>(R, n_clean - first)
