@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -15,7 +16,7 @@
 
 namespace lqcs_b200 {
 
-constexpr size_t kBlockMax = size_t{32} << 20;   // larger blocks are not the pool's
+constexpr size_t kBlockMax = size_t{32} << 20;   // larger blocks are not kept
 constexpr size_t kIdleMax = size_t{256} << 20;
 // Blocks of up to 1 MiB are cut from slabs of 8 MiB: a plan or a program needs a dozen of them.
 constexpr size_t kSlabBlockMax = size_t{1} << 20, kSlab = size_t{8} << 20;
@@ -27,15 +28,20 @@ inline size_t block_size(size_t b) {
     return std::max<size_t>(512, (b + step - 1) / step * step);
 }
 
+// What a buffer for b bytes gets.
+inline size_t capacity(size_t b) { return b <= kBlockMax ? block_size(b) : b; }
+
 template <class Api>
 class BlockPool {
   public:
-    // A block of block_size(b) bytes, b <= kBlockMax; nullptr if the device has no memory left.
-    void* take(int device, size_t b) {
-        const size_t want = block_size(b);
+    // A block of capacity(b) bytes; nullptr if the device has no memory left.  `era` receives the
+    // era it belongs to.
+    void* take(int device, size_t b, uint64_t& era) {
+        const size_t want = capacity(b);
         const bool slab = want <= kSlabBlockMax;
         {
             std::lock_guard<std::mutex> lk(mu_);
+            era = era_;
             if (void* p = find(device, want)) return p;
         }
         void* fresh = Api::allocate(device, slab ? kSlab : want);
@@ -43,68 +49,114 @@ class BlockPool {
             clear();
             fresh = Api::allocate(device, slab ? kSlab : want);
         }
-        if (fresh && slab) {
-            std::lock_guard<std::mutex> lk(mu_);
-            slabs_[device].push_back({static_cast<char*>(fresh), want, 1});
-        }
+        if (!fresh) return nullptr;
+        std::lock_guard<std::mutex> lk(mu_);
+        era = owned_[{device, fresh}] = era_;
+        if (slab) slabs_[device].push_back({static_cast<char*>(fresh), want, 1, era_});
         return fresh;
     }
 
-    // A block of `bytes` from take() comes back.  idle: no work on it is pending, it may be
-    // handed out again.  Otherwise it never is: it is freed with a later block that is idle, or
-    // with its slab once that has no block in use (Api::free waits for the work).
-    void give(int device, void* p, size_t bytes, bool idle) {
-        Frees drop;
+    // A block from take() comes back.  idle: no work on it is pending, it may be handed out
+    // again, unless it is of an earlier era or larger than the pool keeps.  Otherwise it never
+    // is: it is freed with a later block that is idle, or with its slab once that has no block
+    // in use (Api::free waits for the work).
+    void give(int device, void* p, size_t bytes, uint64_t era, bool idle) {
+        std::vector<Free> drop;
         {
             std::lock_guard<std::mutex> lk(mu_);
-            Slab* s = bytes <= kSlabBlockMax ? slab_of(device, p) : nullptr;
+            const bool now = era == era_;
+            Slab* s = bytes > kSlabBlockMax ? nullptr : now ? slab_of(device, p) : retired_slab(device, p, era);
             if (s) --s->live;
-            if (idle) {
+            if (bytes > kBlockMax) {
+                drop.push_back({device, p, era});
+            } else if (!now) {
+                if (!s) later_.push_back({device, p, era});
+                else if (s->live == 0) drop = drop_retired(s);
+            } else if (idle) {
                 idle_[{device, bytes}].push_back(p);
                 idle_bytes_[device] += bytes;
                 if (idle_bytes_[device] > kIdleMax + pinned_[device]) drop = take_idle();
+            } else if (!s) {
+                later_.push_back({device, p, era});
+            }
+            if (idle) {
                 drop.insert(drop.end(), later_.begin(), later_.end());
                 later_.clear();
-            } else if (!s) {
-                later_.emplace_back(device, p);
             }
         }
         release(drop);
     }
 
-    // Frees memory that is not the pool's: at once, or with a later block where that is refused.
-    void discard(int device, void* p) { release({{device, p}}); }
-
-    // Frees the idle blocks and the slabs without a block in use.
-    void clear() {
-        Frees drop;
+    // Frees the idle blocks and the slabs without a block in use.  With `retire` a new era begins:
+    // nothing that was allocated before it is handed out any more.  (After a device reset the
+    // addresses of blocks in use are no longer theirs.)
+    void clear(bool retire = false) {
+        std::vector<Free> drop;
         {
             std::lock_guard<std::mutex> lk(mu_);
             drop = take_idle();
+            if (retire) {
+                ++era_;
+                for (auto& [dev, list] : slabs_) {
+                    for (const Slab& s : list) retired_.emplace_back(dev, s);
+                    list.clear();
+                }
+                idle_.clear();
+                idle_bytes_.clear();
+                pinned_.clear();
+            }
             drop.insert(drop.end(), later_.begin(), later_.end());
             later_.clear();
         }
         release(drop);
     }
 
+    uint64_t era() {
+        std::lock_guard<std::mutex> lk(mu_);
+        return era_;
+    }
+
   private:
-    using Frees = std::vector<std::pair<int, void*>>;
+    struct Free {
+        int device;
+        void* p;
+        uint64_t era;
+    };
     struct Slab {
         char* base;
         size_t used;   // bytes cut so far
         size_t live;   // blocks in use
+        uint64_t era;
     };
     std::mutex mu_;
+    uint64_t era_ = 1;
+    std::map<std::pair<int, void*>, uint64_t> owned_;   // allocations, and their eras
     std::map<std::pair<int, size_t>, std::vector<void*>> idle_;
     std::map<int, size_t> idle_bytes_;
     std::map<int, size_t> pinned_;   // idle bytes the last take_idle left: slabs with blocks in use
     std::map<int, std::vector<Slab>> slabs_;
-    Frees later_;                    // to be freed: work was pending, or Api::free refused
+    std::vector<std::pair<int, Slab>> retired_;   // of earlier eras, with blocks in use
+    std::vector<Free> later_;        // to be freed: work was pending, or Api::free refused
 
     Slab* slab_of(int device, void* p) {
         for (Slab& s : slabs_[device])
             if (p >= s.base && p < s.base + kSlab) return &s;
         return nullptr;
+    }
+    Slab* retired_slab(int device, void* p, uint64_t era) {
+        for (auto& [dev, s] : retired_)
+            if (dev == device && s.era == era && p >= s.base && p < s.base + kSlab) return &s;
+        return nullptr;
+    }
+    // A retired slab whose last block came back.
+    std::vector<Free> drop_retired(const Slab* s) {
+        for (size_t i = 0; i < retired_.size(); ++i) {
+            if (&retired_[i].second != s) continue;
+            const Free f{retired_[i].first, s->base, s->era};
+            retired_.erase(retired_.begin() + static_cast<std::ptrdiff_t>(i));
+            return {f};
+        }
+        return {};
     }
 
     // An idle block, or one cut from a slab.
@@ -130,8 +182,8 @@ class BlockPool {
     }
 
     // Idle blocks and slabs without a block in use, taken out of the pool (to be freed).
-    Frees take_idle() {
-        Frees drop;
+    std::vector<Free> take_idle() {
+        std::vector<Free> drop;
         for (auto& [key, ptrs] : idle_) {
             std::vector<void*> keep;
             for (void* p : ptrs) {
@@ -141,7 +193,7 @@ class BlockPool {
                     continue;
                 }
                 idle_bytes_[key.first] -= key.second;
-                if (!s) drop.emplace_back(key.first, p);
+                if (!s) drop.push_back({key.first, p, era_});
             }
             ptrs.swap(keep);
         }
@@ -149,7 +201,7 @@ class BlockPool {
             std::vector<Slab> keep;
             for (const Slab& s : list) {
                 if (s.live > 0) keep.push_back(s);
-                else drop.emplace_back(dev, s.base);
+                else drop.push_back({dev, s.base, s.era});
             }
             list.swap(keep);
         }
@@ -157,11 +209,19 @@ class BlockPool {
         return drop;
     }
 
-    void release(const Frees& drop) {
-        for (const auto& [dev, p] : drop) {
-            if (Api::free(dev, p)) continue;
+    // Frees what is still the pool's (an address of an earlier era may be a later allocation's).
+    void release(const std::vector<Free>& drop) {
+        for (const Free& f : drop) {
+            {
+                std::lock_guard<std::mutex> lk(mu_);
+                const auto it = owned_.find({f.device, f.p});
+                if (it == owned_.end() || it->second != f.era) continue;
+                owned_.erase(it);
+            }
+            if (Api::free(f.device, f.p)) continue;
             std::lock_guard<std::mutex> lk(mu_);
-            later_.emplace_back(dev, p);
+            owned_.emplace(std::pair{f.device, f.p}, f.era);
+            later_.push_back(f);
         }
     }
 };

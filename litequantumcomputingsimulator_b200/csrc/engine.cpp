@@ -77,7 +77,7 @@ BlockPool<CudaBlocks>& blocks() {   // never destroyed: buffers may be freed dur
 
 }  // namespace
 
-void clear_buffer_pool() { blocks().clear(); }
+void clear_buffer_pool(bool retire) { blocks().clear(retire); }
 
 void DeviceBuffer::release() {
     if (!ptr) return;
@@ -85,22 +85,16 @@ void DeviceBuffer::release() {
     const size_t b = bytes;
     ptr = nullptr;
     bytes = 0;
-    if (b > kBlockMax) blocks().discard(device, p);
-    else blocks().give(device, p, b, CudaBlocks::wait(device, stream));
+    blocks().give(device, p, b, era, b <= kBlockMax && CudaBlocks::wait(device, stream));
 }
 
 void DeviceBuffer::ensure(size_t b) {
     if (b <= bytes) return;
     release();
     cuda_check(cudaGetDevice(&device), "cudaGetDevice");
-    if (b <= kBlockMax) {
-        ptr = blocks().take(device, b);
-    } else if (!(ptr = CudaBlocks::allocate(device, b))) {   // once more without the idle blocks
-        clear_buffer_pool();
-        ptr = CudaBlocks::allocate(device, b);
-    }
+    ptr = blocks().take(device, b, era);
     if (!ptr) cuda_check(cudaErrorMemoryAllocation, "cudaMalloc");
-    bytes = b <= kBlockMax ? block_size(b) : b;
+    bytes = capacity(b);
 }
 
 int device_sm_count() {
@@ -706,6 +700,7 @@ struct PooledBuffer {
     int device;
     size_t bytes;
     void* ptr;
+    uint64_t era;
 };
 // Never destroyed: states may be freed during process exit, after static destructors ran.
 std::mutex& pool_mu() {
@@ -719,16 +714,20 @@ std::vector<PooledBuffer>& pool() {   // oldest first
 constexpr size_t kPoolMaxBytes = size_t{1} << 30;
 constexpr size_t kPoolEntries = 4;
 
-void* pool_take(int device, size_t bytes) {
+// A kept buffer of this size for `b`; false if there is none.
+bool pool_take(int device, size_t bytes, DeviceBuffer& b) {
     std::lock_guard<std::mutex> lk(pool_mu());
     for (auto it = pool().begin(); it != pool().end(); ++it) {
         if (it->device == device && it->bytes == bytes) {
-            void* p = it->ptr;
+            b.ptr = it->ptr;
+            b.bytes = bytes;
+            b.device = device;
+            b.era = it->era;
             pool().erase(it);
-            return p;
+            return true;
         }
     }
-    return nullptr;
+    return false;
 }
 
 }  // namespace
@@ -739,28 +738,27 @@ void clear_state_pool() {
         std::lock_guard<std::mutex> lk(pool_mu());
         drop.swap(pool());
     }
-    for (const PooledBuffer& b : drop) blocks().discard(b.device, b.ptr);
+    for (const PooledBuffer& b : drop) blocks().give(b.device, b.ptr, b.bytes, b.era, false);
 }
 
 void pool_return(lqcs_state& st) {
     // (smaller ones are the block pool's)
     if (!st.amps.ptr || st.amps.bytes <= kBlockMax || st.amps.bytes > kPoolMaxBytes) return;
+    if (st.amps.era != blocks().era()) return;   // allocated before lqcs_release_caches: not kept
     // the buffer is reused only after this state's work on it has finished
     if (!CudaBlocks::wait(st.device, st.stream)) return;
-    void* evict = nullptr;
-    int evict_dev = 0;
+    PooledBuffer evict{};
     {
         std::lock_guard<std::mutex> lk(pool_mu());
         if (pool().size() >= kPoolEntries) {
-            evict = pool().front().ptr;
-            evict_dev = pool().front().device;
+            evict = pool().front();
             pool().erase(pool().begin());
         }
-        pool().push_back({st.device, st.amps.bytes, st.amps.ptr});
+        pool().push_back({st.device, st.amps.bytes, st.amps.ptr, st.amps.era});
     }
     st.amps.ptr = nullptr;
     st.amps.bytes = 0;
-    if (evict) blocks().discard(evict_dev, evict);
+    if (evict.ptr) blocks().give(evict.device, evict.ptr, evict.bytes, evict.era, false);
 }
 
 std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t stream) {
@@ -787,11 +785,7 @@ std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t s
     st->stream = st->amps.stream = st->scratch.stream = st->sample_scratch.stream = stream;
     st->ctx = make_ctx(stream);
     const size_t bytes = sizeof(double2) * st->len() * batch;
-    if (void* p = pool_take(st->device, bytes)) {
-        st->amps.ptr = p;
-        st->amps.bytes = bytes;
-        st->amps.device = st->device;
-    } else {
+    if (!pool_take(st->device, bytes, st->amps)) {
         try {
             st->amps.ensure(bytes);
         } catch (const Error& e) {

@@ -27,12 +27,13 @@ struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
+    uint64_t era = 0;   // the pool's when it was allocated
     cudaStream_t stream = nullptr;
     explicit DeviceBuffer(cudaStream_t s = nullptr) : stream(s) {}
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
     DeviceBuffer(DeviceBuffer&& o) noexcept
-        : ptr(o.ptr), bytes(o.bytes), device(o.device), stream(o.stream) {
+        : ptr(o.ptr), bytes(o.bytes), device(o.device), era(o.era), stream(o.stream) {
         o.ptr = nullptr;
         o.bytes = 0;
     }
@@ -42,6 +43,7 @@ struct DeviceBuffer {
             ptr = o.ptr;
             bytes = o.bytes;
             device = o.device;
+            era = o.era;
             stream = o.stream;
             o.ptr = nullptr;
             o.bytes = 0;
@@ -126,8 +128,9 @@ uint32_t default_fusion_width();
 void clear_program_cache();
 // Free the amplitude buffers kept for new states of the same size.
 void clear_state_pool();
-// Free the idle blocks of the buffer pool.
-void clear_buffer_pool();
+// Free the idle blocks of the buffer pool; with `retire` what is in use leaves the pool too (each
+// block is freed when its buffer is, none is handed out again).
+void clear_buffer_pool(bool retire = false);
 // The compiled program of a gate list: one of the last few circuits' or a new one.
 std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
                                               const FusionConfig& fc, cudaStream_t stream);

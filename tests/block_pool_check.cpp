@@ -14,7 +14,7 @@ struct Fake {
     static inline std::set<void*> held;
     static inline size_t allocations = 0, bad_frees = 0;
     static inline bool refuse_free = false, out_of_memory = false;
-    static void reset() {
+    static void reset() {   // as a device reset: every address is free again
         next = reinterpret_cast<char*>(size_t{1} << 40);   // addresses only, never read
         held.clear();
         allocations = bad_frees = 0;
@@ -34,8 +34,15 @@ struct Fake {
         return true;
     }
 };
-using Pool = lqcs_b200::BlockPool<Fake>;
 using lqcs_b200::block_size;
+
+struct Pool : lqcs_b200::BlockPool<Fake> {
+    using Base = lqcs_b200::BlockPool<Fake>;
+    uint64_t last = 0;   // era of the block taken last
+    void* take(int device, size_t b) { return Base::take(device, b, last); }
+    void give(int device, void* p, size_t bytes, bool idle) { Base::give(device, p, bytes, era(), idle); }
+    using Base::give;
+};
 
 void expect(bool ok, const char* what) {
     if (ok) return;
@@ -67,11 +74,13 @@ void pending_slab_is_freed() {
 void pending_large() {
     Pool pool;
     const size_t mib2 = size_t{2} << 20;
+    const size_t mib64 = size_t{64} << 20;
     void* a = pool.take(0, mib2);
     void* b = pool.take(0, mib2);
+    void* c = pool.take(0, mib64);
     Fake::refuse_free = true;   // as during a capture
     pool.give(0, a, mib2, false);
-    pool.discard(0, Fake::allocate(0, 64));
+    pool.give(0, c, mib64, false);
     expect(Fake::held.size() == 3, "nothing can be freed now");
     Fake::refuse_free = false;
     pool.give(0, b, mib2, true);
@@ -91,10 +100,61 @@ void bounds() {
     expect(pool.take(0, size_t{32} << 20) != nullptr, "idle blocks were not given up");
 }
 
+// What was allocated before the caches were released is not handed out again.  Without a device
+// reset in between it is freed with its last block; after one its addresses may be another's.
+void released_slab() {
+    Pool pool;
+    void* a = pool.take(0, 1000);
+    void* b = pool.take(0, 1000);
+    const uint64_t era = pool.last;
+    pool.clear(true);
+    void* c = pool.take(0, 1000);
+    expect(Fake::allocations == 2, "a block was cut from a retired slab");
+    pool.give(0, a, block_size(1000), era, true);
+    expect(pool.take(0, 1000) != a, "a block of a retired slab was handed out");
+    expect(Fake::held.size() == 2, "a retired slab with a block in use stays");
+    pool.give(0, b, block_size(1000), era, true);
+    expect(Fake::held.size() == 1 && Fake::bad_frees == 0, "the retired slab was not freed");
+    pool.give(0, c, block_size(1000), true);
+    expect(pool.take(0, 1000) == c, "a block of this era is handed out again");
+}
+void released_large() {
+    Pool pool;
+    const size_t mib2 = size_t{2} << 20;
+    void* a = pool.take(0, mib2);
+    const uint64_t era = pool.last;
+    pool.clear(true);
+    pool.give(0, a, mib2, era, true);
+    expect(pool.take(0, mib2) != a, "a block from before the release was handed out");
+}
+void reset_device() {
+    Pool pool;
+    const size_t mib2 = size_t{2} << 20;
+    void* a = pool.take(0, 1000);
+    void* b = pool.take(0, 1000);
+    void* big = pool.take(0, mib2);
+    const uint64_t era = pool.last;
+    Fake::reset();
+    pool.clear(true);
+    void* c = pool.take(0, 1000);   // the same addresses again
+    expect(c == a, "the fake device hands out its first address again");
+    pool.give(0, a, block_size(1000), era, true);
+    pool.give(0, b, block_size(1000), era, true);
+    expect(Fake::held.count(c) == 1, "a slab of this era was freed as an old one");
+    void* d = pool.take(0, 1000);
+    expect(d != c && d != nullptr, "a block in use was handed out twice");
+    void* big2 = pool.take(0, mib2);
+    expect(big2 == big, "the fake device hands out the same addresses");
+    pool.give(0, big, mib2, era, true);
+    expect(Fake::held.count(big2) == 1, "a block of this era was freed as an old one");
+    expect(pool.take(0, mib2) != big2, "a block in use was handed out twice");
+}
+
 }  // namespace
 
 int main() {
-    for (auto* check : {pending_small, pending_slab_is_freed, pending_large, bounds}) {
+    for (auto* check : {pending_small, pending_slab_is_freed, pending_large, bounds, released_slab,
+                        released_large, reset_device}) {
         Fake::reset();
         check();
     }
