@@ -775,7 +775,12 @@ std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t s
     const bool small = n <= 40 && (static_cast<double>(batch) * std::ldexp(16.0, static_cast<int>(n))) <=
                                       static_cast<double>(kBlockMax);
     if (!small) {
-        const uint32_t cap = max_qubits_on_device(batch);
+        uint32_t cap = max_qubits_on_device(batch);
+        if (n > cap && n <= 40) {   // once more without what lies idle
+            clear_state_pool();
+            clear_buffer_pool();
+            cap = max_qubits_on_device(batch);
+        }
         if (n > cap || n > 40) too_large(cap);
     }
     auto st = std::make_unique<lqcs_state>();

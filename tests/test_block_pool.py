@@ -75,3 +75,23 @@ def test_frees_beside_captures():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.gpu
+def test_idle_blocks_make_room_for_a_state():
+    """A state that fits only where the idle blocks lie is not refused."""
+    import torch
+    A.release_caches()
+    small = [lq.Statevector(21) for _ in range(8)]   # 8 blocks of 32 MiB
+    del small                                        # idle now
+    free, _total = torch.cuda.mem_get_info()
+    need = 16 << 25                                  # 512 MiB
+    filler = torch.empty(free - need + (128 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        sv = lq.Statevector(25)
+        assert sv.norm() == 1.0
+        del sv
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+        A.release_caches()
