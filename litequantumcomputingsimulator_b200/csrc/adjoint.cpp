@@ -17,7 +17,6 @@
 #include <memory>
 #include <mutex>
 #include <numbers>
-#include <set>
 
 #include "adj_pass.cuh"
 #include "engine.hpp"
@@ -322,14 +321,10 @@ int env_or(const char* name, int dflt) {
     return e ? std::atoi(e) : dflt;
 }
 
-// Everything one (circuit, Hamiltonian, resident batch) needs on the device, kept between
-// calls: the fixed gates and their inverses, the two resident state batches, the Hamiltonian
-// terms and the per-set buffers, on a stream of its own.  A call only uploads the new
-// (cos, sin) tables, so the launch sequence of a batch of nb sets never changes: it is
-// captured once as a CUDA graph and replayed (LQCS_GRAPHS=0: launched directly).
 // The two resident state batches of a plan: scratch of one call.  Plans of one shape whose
-// batches are large (above 32 MiB: one call fills the GPU) share a pair, so a new plan of a known
-// shape allocates none and sixteen plans hold little; `mu` is held during a call.
+// batches are large (one call fills the GPU) share a pair, so a new plan of a known shape allocates
+// none and sixteen plans hold little; `mu` is held during a call.
+constexpr size_t kSharedPairBytes = size_t{32} << 20;   // above: large
 struct StatePair {
     int device = 0;
     uint32_t n = 0, R = 0;
@@ -338,6 +333,11 @@ struct StatePair {
     size_t bytes() const { return 2 * static_cast<size_t>(R) * (size_t{16} << n); }
 };
 
+// Everything one (circuit, Hamiltonian, resident batch) needs on the device, kept between
+// calls: the fixed gates and their inverses, the two resident state batches, the Hamiltonian
+// terms and the per-set buffers, on a stream of its own.  A call only uploads the new
+// (cos, sin) tables, so the launch sequence of a batch of nb sets never changes: it is
+// captured as a CUDA graph after a few calls and replayed (LQCS_GRAPHS=0: launched directly).
 struct AdjointPlan {
     uint64_t key = 0;
     uint32_t n = 0, R = 0;
@@ -357,7 +357,7 @@ struct AdjointPlan {
     cudaStream_t stream = nullptr;
     // (2 nb + with gradients) -> (graph, kernels)
     std::map<uint32_t, std::pair<cudaGraphExec_t, uint64_t>> graphs;
-    std::set<uint32_t> seen;   // keys that have run
+    std::map<uint32_t, uint32_t> direct_runs;   // of the same keys, before their capture
 
     AdjointPlan() = default;
     AdjointPlan(const AdjointPlan&) = delete;
@@ -511,6 +511,14 @@ struct AdjointPlan {
         d_rot_part.ensure(sizeof(double) * max_ops * R * (uint64_t{1} << (n - mb)));
     }
 
+    // Runs of a batch size that are launched directly before its graph is captured.  Capturing and
+    // instantiating cost as much as many replays save: 0.13 to 0.6 ms against 0.02 to 0.07 ms a call
+    // (9 to 14 qubits, states of at most 32 MiB), and 1 to 40 ms (the instantiation's
+    // allocations stall) against 0.1 to 0.2 ms where the batch fills the GPU (18 qubits, 16 sets:
+    // 1.70 direct, 1.60 replayed; 16 qubits, 256 sets: 16.0 and 15.8).  So a few calls never pay
+    // for a graph, and a long loop gets it.
+    uint32_t runs_before_capture() const { return states->bytes() > kSharedPairBytes ? 64 : 8; }
+
     void run(uint32_t nb, bool grads = true) {
         const char* e = std::getenv("LQCS_GRAPHS");
         if (e && e[0] == '0') {
@@ -520,8 +528,7 @@ struct AdjointPlan {
         const uint32_t key = 2 * nb + (grads ? 1u : 0u);
         auto it = graphs.find(key);
         bool fresh = false;
-        if (it == graphs.end() && seen.insert(key).second) {
-            // a batch size's first call: capturing and instantiating costs more than it saves
+        if (it == graphs.end() && ++direct_runs[key] <= runs_before_capture()) {
             enqueue(nb, grads);
             return;
         }
@@ -618,7 +625,7 @@ std::shared_ptr<AdjointPlan> adjoint_plan(const std::vector<GateDesc>& tmpl, con
         }
     std::shared_ptr<StatePair> shared;
     const size_t need = 2 * static_cast<size_t>(R) * (size_t{16} << n);
-    if (need > (size_t{32} << 20))
+    if (need > kSharedPairBytes)
         for (const auto& p : g_plans)
             if (p->states->device == dev && p->n == n && p->R == R) shared = p->states;
     auto held = [&] {

@@ -1,0 +1,45 @@
+"""When the batched adjoint captures its launches as a CUDA graph: not in the first calls (a
+capture costs as much as many replays save), and then once; replays with new parameters give
+what direct launches give, bit for bit.
+
+Small plans are captured on the ninth call of a batch size, plans whose states exceed 32 MiB on the
+65th.  CUDA runtime calls are counted with torch's profiler."""
+import numpy as np
+import pytest
+
+import litequantumcomputingsimulator_b200 as lq
+from litequantumcomputingsimulator_b200 import algorithms as A
+from litequantumcomputingsimulator_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def runtime_calls(f):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.zeros(1, device="cuda")
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    return {e.key: e.count for e in prof.key_averages()}
+
+
+@pytest.mark.parametrize("n,sets,before", [(6, 2, 8), (9, 3, 8), (12, 4, 8), (15, 48, 64)])
+def test_captured_after_several_calls(monkeypatch, n, sets, before):
+    gates = 12
+    pc, _ = W.random_pauli_ansatz(n, gates, n)
+    ham = W.random_hamiltonian(n, 10, n + 1)
+    params = [W.random_parameter_sets(gates, sets, 100 + k) for k in range(before + 3)]
+    monkeypatch.setenv("LQCS_GRAPHS", "0")
+    want = [A.adjoint_gradient(ham, pc, p) for p in params]
+    monkeypatch.delenv("LQCS_GRAPHS")
+    A.release_caches()
+    got = []
+    direct = runtime_calls(lambda: got.extend(A.adjoint_gradient(ham, pc, p) for p in params[:before]))
+    replays = runtime_calls(lambda: got.extend(A.adjoint_gradient(ham, pc, p) for p in params[before:]))
+    A.release_caches()
+    for (e, g), (we, wg) in zip(got, want):
+        assert np.array_equal(e, we) and np.array_equal(g, wg)
+    assert direct.get("cudaLaunchKernel", 0) > 0, direct   # the profiler sees the engine's calls
+    assert direct.get("cudaGraphLaunch", 0) == 0, direct
+    assert replays.get("cudaGraphLaunch", 0) == 3, replays
