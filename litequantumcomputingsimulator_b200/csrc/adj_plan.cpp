@@ -147,9 +147,13 @@ std::vector<AdjPass> plan_adjoint_passes(const std::vector<AdjRotation>& rots, u
         for (uint32_t q = 0; q < 3; ++q) space.add(uint64_t{1} << q);
         std::vector<AdjRotation> cur, rest;
         uint32_t layouts = 1, in_layout = 0;   // an upper bound on the layouts taken so far
-        for (const AdjRotation& r : pend) {
-            bool ok = cur.size() < most && layouts < kAdjMaxLayouts &&
-                      (space.v.size() < m || space.contains(r.x));
+        for (size_t i = 0; i < pend.size(); ++i) {
+            const AdjRotation& r = pend[i];
+            if (cur.size() == most) {   // full
+                rest.insert(rest.end(), pend.begin() + static_cast<std::ptrdiff_t>(i), pend.end());
+                break;
+            }
+            bool ok = layouts < kAdjMaxLayouts && (space.v.size() < m || space.contains(r.x));
             for (size_t k = 0; !any_order && ok && k < rest.size(); ++k) ok = commute(r, rest[k]);
             if (!ok) {
                 rest.push_back(r);

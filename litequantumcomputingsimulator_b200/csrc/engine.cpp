@@ -990,16 +990,29 @@ std::vector<double> expectation_terms(lqcs_state& st, const std::vector<PauliMas
     // terms of one x mask side by side: they share a layout
     std::stable_sort(list.begin(), list.end(),
                      [](const AdjRotation& a, const AdjRotation& b) { return a.x < b.x; });
+    // A bounded number of terms at a time: planning passes takes (terms) * (passes), and a term's
+    // partial sums up to 4.7 KB (a block each on 148 SMs).  The device runs one group while the host
+    // plans the next; with all terms in one group, 20000 diagonal ones on 15 qubits took 45 ms
+    // instead of 16, 3000 random ones on 24 qubits 33 instead of 28.
+    constexpr uint32_t kGroup = 1024;
     const uint32_t blocks = expect_blocks(st.ctx, st.n);
-    st.scratch.ensure(sizeof(double) * count * (size_t{blocks} + 1));
-    double* part = st.scratch.as<double>();
-    double* d_out = part + static_cast<size_t>(count) * blocks;
-    for (const AdjPass& p : plan_adjoint_passes(list, st.n, kExpectTileBits, 4, true, kExpectTerms))
-        launch_expect_pass(st.ctx, st.d(), st.n, p, part);
-    launch_expect_sum(st.ctx, st.n, count, part, d_out);
-    cuda_check(cudaMemcpyAsync(vals.data(), d_out, sizeof(double) * count, cudaMemcpyDeviceToHost,
+    st.scratch.ensure(sizeof(double) * (count + size_t{blocks} * std::min(count, kGroup)));
+    double* d_out = st.scratch.as<double>();   // in the sorted order
+    double* part = d_out + count;
+    std::vector<AdjRotation> group;
+    for (uint32_t first = 0; first < count; first += kGroup) {
+        const uint32_t n_terms = std::min(kGroup, count - first);
+        group.assign(list.begin() + first, list.begin() + first + n_terms);
+        for (uint32_t t = 0; t < n_terms; ++t) group[t].param = t;
+        for (const AdjPass& p : plan_adjoint_passes(group, st.n, kExpectTileBits, 4, true, kExpectTerms))
+            launch_expect_pass(st.ctx, st.d(), st.n, p, part);
+        launch_expect_sum(st.ctx, st.n, n_terms, part, d_out + first);
+    }
+    std::vector<double> sorted(count);
+    cuda_check(cudaMemcpyAsync(sorted.data(), d_out, sizeof(double) * count, cudaMemcpyDeviceToHost,
                                st.stream), "D2H expectations");
     st.sync();
+    for (uint32_t t = 0; t < count; ++t) vals[list[t].param] = sorted[t];
     return vals;
 }
 

@@ -43,3 +43,24 @@ def test_expectation_terms(n, count):
     want = [plain(psi, p) for p in paulis]
     assert np.max(np.abs(got - np.array(want))) < 1e-12
     assert np.array_equal(A.expectation_terms(sv, paulis), got)   # fixed order
+
+
+@pytest.mark.parametrize("n,letters", [(15, "IZ"), (16, "IXYZ"), (20, "IZ")])
+def test_many_terms_in_bounded_memory(n, letters):
+    """More terms than are planned and summed at a time (1024), in every order of X masks; the scratch
+    does not grow with the number of terms times blocks (20000 * 512 * 8 bytes = 78 MiB)."""
+    import torch
+    rng = np.random.default_rng(n)
+    count = 20000 if letters == "IZ" else 2600
+    paulis = ["".join(letters[int(v)] for v in rng.integers(0, len(letters), n)) for _ in range(count)]
+    sv = lq.Statevector.from_numpy(W.gaussian_state(n, n))
+    A.release_caches()
+    A.expectation_terms(sv, paulis[:1])
+    free, _total = torch.cuda.mem_get_info()
+    got = A.expectation_terms(sv, paulis)
+    assert free - torch.cuda.mem_get_info()[0] <= 32 << 20
+    some = list(range(0, count, 97)) + [1023, 1024, count - 1]
+    # the same terms with others about them: another pass, the same sum up to rounding
+    want = np.concatenate([A.expectation_terms(sv, [paulis[k] for k in some[i:i + 50]])
+                           for i in range(0, len(some), 50)])
+    assert np.max(np.abs(got[some] - want)) < 1e-12
