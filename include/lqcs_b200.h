@@ -484,7 +484,8 @@ uint64_t lqcs_kernel_launch_count(void);
  * all tiles, 0 = none, 3 = the double-buffered kernel (LQCS_REG_PIPE=1; 2^11- and
  * 2^12-amplitude tiles); + 8 leaves out the barrier a relabelling pass puts between its
  * loads and stores.  *n_races counts racing accesses; `report` (capacity report_cap)
- * receives the first.  Fails if a gate does not run inside a register pass. */
+ * receives the first, or, if there is none, how many of the passes are in rotation form.  Fails if
+ * a gate does not run inside a register pass. */
 int lqcs_debug_emulate_register_passes(uint32_t n_qubits, const lqcs_instruction* insts,
                                        uint64_t n_insts, uint64_t grid, int32_t sync_tiles,
                                        double* state, uint64_t race_ctas, uint64_t* n_passes,

@@ -645,7 +645,7 @@ void emulate_register_program(uint32_t n, const lqcs_instruction* insts, uint64_
     if (!cfg.reg) invalid("register tile emulation: register passes are switched off");
     const auto items = plan_tiles(gates, n, cfg);
     RaceLog log;
-    uint64_t passes = 0;
+    uint64_t passes = 0, rot = 0;
     std::vector<cd> next;
     AmpLog amps;
     if (state) {
@@ -681,10 +681,13 @@ void emulate_register_program(uint32_t n, const lqcs_instruction* insts, uint64_
             std::memcpy(state, next.data(), sizeof(cd) * next.size());
         }
         ++passes;
+        rot += rp.rot;
     }
     *n_passes = passes;
     *n_races = log.races;
-    if (report) *report = log.first;
+    if (report)
+        *report = log.races ? log.first
+                            : std::to_string(rot) + " of " + std::to_string(passes) + " passes in rotation form";
 }
 
 }  // namespace lqcs_b200

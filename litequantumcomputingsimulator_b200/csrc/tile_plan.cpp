@@ -1611,6 +1611,10 @@ struct Emitted {
 // its tile bits, and then goes out in one table with everything else that fits beside it.
 class DiagonalPool {
   public:
+    // compact: strided tables of at most six bits (64 entries) where an expanded one has up to
+    // 136: slower to read (an address per entry), for passes whose matrices would outgrow their
+    // stage.
+    explicit DiagonalPool(bool compact) : compact_(compact) {}
     static bool takes(const LocalOp& o) {
         if (o.kind == kTilePhase)
             return __builtin_popcount(o.lmask) <= static_cast<int>(kRegMaxDiag);
@@ -1641,6 +1645,7 @@ class DiagonalPool {
         uint32_t bits;
     };
     std::vector<Item> items_;
+    bool compact_;
 
     static uint32_t bits_of(const LocalOp& o) { return o.kind == kTilePhase ? o.lmask : target_mask(o); }
     static int width(uint32_t bits) { return __builtin_popcount(bits); }
@@ -1662,9 +1667,9 @@ class DiagonalPool {
     // Tile bits of the next table: whole components of joined bits while they fit, first those
     // with a bit of `touch`; if the first is too wide, as much of it as fits.  Fitting: at most
     // three thread bits beside the register bits S (an expanded table); with gated phases about,
-    // or where nothing fits so, six bits (a strided one, which a tile may build).
+    // where nothing fits so, or compact, six bits (a strided one, which a tile may build).
     uint32_t group(uint32_t touch, uint32_t S) const {
-        bool gated = false;
+        bool gated = compact_;
         for (const Item& it : items_) gated |= it.op->kind == kTilePhase && it.op->gcmask != 0;
         for (int strided = gated ? 1 : 0; strided < 2; ++strided) {
             auto fits = [&](uint32_t bits) {
@@ -1694,7 +1699,7 @@ class DiagonalPool {
     void emit(uint32_t u, Emitted& e, const RegLayout& ly, uint32_t S, uint32_t m) {
         RegOp r{};
         std::vector<uint32_t> bits;
-        const bool narrow_enough = width(u & ~S) <= static_cast<int>(kRegTableThreadBits);
+        const bool narrow_enough = !compact_ && width(u & ~S) <= static_cast<int>(kRegTableThreadBits);
         for (uint8_t& l : r.loc) l = 31;
         for (uint32_t i = 0; i < m - kRegBits; ++i)
             if ((u >> ly.tpos[i]) & 1) {
@@ -1869,6 +1874,12 @@ class PendingSigns {
     bool used_ = false;
 };
 
+// How the records of a pass in rotation form are written: with bits stored negated, with
+// compact tables.
+struct RotVariant {
+    bool flips = true, compact = false;
+};
+
 // Records and matrices of the schedule `seq` for the operations of one state.  In rotation
 // form the operations of one layout go out in the order that leaves diagonals waiting longest:
 // whatever mixes a bit that nothing waits on goes first, and a table is emitted only when
@@ -1879,13 +1890,13 @@ void emit_schedule(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
                    const std::vector<uint8_t>& mma,
                    const std::vector<std::pair<int, uint32_t>>& seq,
                    const std::vector<RegLayout>& lays, const std::vector<Lay>& keys, uint32_t m,
-                   const std::vector<uint32_t>& store_q, bool rot, bool flips, Emitted& e) {
-    DiagonalPool pool;
+                   const std::vector<uint32_t>& store_q, bool rot, RotVariant variant, Emitted& e) {
+    DiagonalPool pool(variant.compact);
     std::deque<LocalOp> scales;   // diagonals of mirrored rotations (the pool keeps pointers)
     uint32_t cur = 0;
     if (rot) e.mats.emplace_back(0.0, 0.0);   // what the store undoes
     // bits that controls of records look at are never stored negated
-    uint32_t keep = flips ? 0u : ~0u;
+    uint32_t keep = variant.flips ? 0u : ~0u;
     for (const LocalOp& o : ops) {
         e.per_state |= o.variant;
         if (!DiagonalPool::takes(o) && o.kind != kTilePauli) {
@@ -2018,17 +2029,21 @@ void emit_schedule(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
     }
 }
 
+// selects: set if some block takes one of several matrices, so that fewer selector qubits would
+// leave fewer matrices.
 bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates,
-                        const TileConfig& cfg, uint32_t max_select, bool rot, bool flips, RegPass& pass,
+                        const TileConfig& cfg, uint32_t max_select, bool rot, RegPass& pass,
                         std::vector<RegOp>& ops_out, std::vector<RegLayout>& layouts_out,
                         std::vector<cd>& mats_out, double* flops_per_amp,
-                        const std::vector<std::vector<std::array<cd, 4>>>* state_slots) {
+                        const std::vector<std::vector<std::array<cd, 4>>>* state_slots, bool& selects) {
     const uint32_t m = cfg.L + static_cast<uint32_t>(item.hbits.size());
     const std::vector<std::array<cd, 4>>* slots0 =
         state_slots && !state_slots->empty() ? &(*state_slots)[0] : nullptr;
     std::vector<uint32_t> store_q;
     const std::vector<LocalOp> ops =
         pass_local_ops(item, gates, cfg, max_select, slots0, kRegMaxDiag, true, &store_q, true, rot);
+    selects = false;
+    for (const LocalOp& o : ops) selects |= !o.sel.empty();
     for (const LocalOp& o : ops)
         if (o.kind != kTilePhase && o.kind != kTilePauli && o.kind != kTileRot &&
             o.lt.size() > (o.kind == kTileDense ? kRegMaxK : kRegMaxDiag))
@@ -2167,23 +2182,14 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
         }
     }
 
-    // records and the first state's matrices
-    Emitted first;
-    emit_schedule(ops, use, mma, seq, lays, lay_keys, m, store_q, rot, flips, first);
-    if (first.failed) return false;
-    bool flipped = first.flipped != 0;
-    const std::vector<RegOp>& rec = first.rec;
-    std::vector<cd>& mats = first.mats;
-    const std::vector<uint32_t>& dyn_rec = first.dyn_rec;
-    const uint32_t dyn_entries = first.dyn_entries;
-    if (rec.size() > kRegMaxRecords || lays.size() > kRegMaxLayouts || mats.size() > kRegMaxMatrix ||
-        dyn_rec.size() > kRegMaxDyn || dyn_entries > kRegMaxDynEntries)
-        return false;
-    const size_t n_mat = mats.size();
-    // every further state: same records, its own slot matrices
+    // records and every state's matrices; the states share the records
+    struct State {
+        std::vector<LocalOp> ops;
+        size_t same;   // the state with the same matrices in all of the pass's slots: most often
+                       // there is no error at all, and such states share the work
+    };
+    std::vector<State> states;   // 1 and up
     if (state_slots) {
-        // (states with the same matrices in all of the pass's slots, most often no error at all,
-        // share the work)
         std::map<std::string, size_t> known;   // slot matrices -> the state lowered for them
         auto key_of = [&](size_t b) {
             std::string k;
@@ -2196,26 +2202,60 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
         known.emplace(key_of(0), 0);
         for (size_t b = 1; b < state_slots->size(); ++b) {
             const auto [same, fresh] = known.emplace(key_of(b), b);
-            if (!fresh) {
-                mats.resize(mats.size() + n_mat);
-                std::copy_n(mats.begin() + static_cast<long>(same->second * n_mat), n_mat,
-                            mats.end() - static_cast<long>(n_mat));
-                continue;
-            }
+            states.push_back({{}, same->second});
+            if (!fresh) continue;
             std::vector<uint32_t> store_b;
-            const std::vector<LocalOp> ob = pass_local_ops(item, gates, cfg, max_select,
-                                                           &(*state_slots)[b], kRegMaxDiag, true,
-                                                           &store_b, true, rot);
+            states.back().ops = pass_local_ops(item, gates, cfg, max_select, &(*state_slots)[b],
+                                               kRegMaxDiag, true, &store_b, true, rot);
+            const std::vector<LocalOp>& ob = states.back().ops;
             if (ob.size() != ops.size() || store_b != store_q) return false;
             for (size_t i = 0; i < ops.size(); ++i)
                 if (!same_shape(ops[i], ob[i])) return false;
-            Emitted eb;
-            emit_schedule(ob, use, mma, seq, lays, lay_keys, m, store_q, rot, flips, eb);
-            flipped |= eb.flipped != 0;
-            if (eb.failed || eb.mats.size() != n_mat || eb.rec.size() != rec.size()) return false;
-            mats.insert(mats.end(), eb.mats.begin(), eb.mats.end());
         }
     }
+    Emitted first;
+    bool flipped = false;
+    size_t n_mat = 0;
+    enum Fit { kFits, kMatrices, kLimits, kForm };   // too many matrices, records, ...; a state whose
+                                                     // operations these records cannot express
+    auto emit = [&](RotVariant v) {
+        first = Emitted{};
+        emit_schedule(ops, use, mma, seq, lays, lay_keys, m, store_q, rot, v, first);
+        if (first.failed) return kForm;
+        if (first.rec.size() > kRegMaxRecords || lays.size() > kRegMaxLayouts ||
+            first.dyn_rec.size() > kRegMaxDyn || first.dyn_entries > kRegMaxDynEntries)
+            return kLimits;
+        if (first.mats.size() > kRegMaxMatrix) return kMatrices;
+        flipped = first.flipped != 0;
+        n_mat = first.mats.size();
+        std::vector<cd>& mats = first.mats;
+        for (size_t b = 1; b <= states.size(); ++b) {
+            const State& st = states[b - 1];
+            if (st.same != b) {
+                mats.resize(mats.size() + n_mat);
+                std::copy_n(mats.begin() + static_cast<long>(st.same * n_mat), n_mat,
+                            mats.end() - static_cast<long>(n_mat));
+                continue;
+            }
+            Emitted eb;
+            emit_schedule(st.ops, use, mma, seq, lays, lay_keys, m, store_q, rot, v, eb);
+            flipped |= eb.flipped != 0;
+            if (eb.failed || eb.mats.size() != n_mat || eb.rec.size() != first.rec.size()) return kForm;
+            mats.insert(mats.end(), eb.mats.begin(), eb.mats.end());
+        }
+        return kFits;
+    };
+    Fit fit = emit({});
+    if (rot && fit == kMatrices) fit = emit({true, true});
+    if (rot && fit == kForm) {   // without negated bits
+        fit = emit({false, false});
+        if (fit == kMatrices) fit = emit({false, true});
+    }
+    if (fit != kFits) return false;
+    const std::vector<RegOp>& rec = first.rec;
+    const std::vector<cd>& mats = first.mats;
+    const std::vector<uint32_t>& dyn_rec = first.dyn_rec;
+    const uint32_t dyn_entries = first.dyn_entries;
     pass = RegPass{};
     pass.L = cfg.L;
     pass.h = static_cast<uint32_t>(item.hbits.size());
@@ -2279,15 +2319,17 @@ bool lower_pass_reg(const PlanItem& item, const std::vector<GateDesc>& gates,
                     const std::vector<std::vector<std::array<cd, 4>>>* state_slots) {
     const uint32_t m = cfg.L + static_cast<uint32_t>(item.hbits.size());
     if (m < kRegMinBits || m > kRegMaxBits || item.hbits.size() > kTileMaxHigh) return false;
-    // fewer selector qubits when the matrices of a pass outgrow their shared-memory stage
-    // or, where they still do, or where the states of a batch differ in form (a noise matrix
-    // that has no rotation form in some state), dense operations with merged diagonals; form 2:
-    // rotation form, 1: rotation form without negated bits
-    for (int form = uses_rotation_form(cfg) ? 2 : 0; form >= 0; --form)
-        for (int sel = static_cast<int>(kRegMaxSelect); sel >= 0; --sel)
-            if (lower_pass_reg_sel(item, gates, cfg, static_cast<uint32_t>(sel), form > 0, form == 2,
-                                   pass, ops_out, layouts_out, mats_out, flops_per_amp, state_slots))
+    // fewer selector qubits when the matrices of a pass outgrow their shared-memory stage (where
+    // it has any); where they still do, or where the states of a batch differ in form (a noise
+    // matrix that has no rotation form in some state), dense operations with merged diagonals
+    for (int rot = uses_rotation_form(cfg) ? 1 : 0; rot >= 0; --rot)
+        for (int sel = static_cast<int>(kRegMaxSelect); sel >= 0; --sel) {
+            bool selects = false;
+            if (lower_pass_reg_sel(item, gates, cfg, static_cast<uint32_t>(sel), rot != 0, pass, ops_out,
+                                   layouts_out, mats_out, flops_per_amp, state_slots, selects))
                 return true;
+            if (!selects) break;
+        }
     return false;
 }
 
