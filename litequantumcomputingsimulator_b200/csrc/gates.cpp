@@ -53,32 +53,61 @@ double param(const GateDesc& g, size_t i) {
     return g.params[i];
 }
 
-// Apply a dense gate (matrix f on local positions pos[0..m-1] of a k-bit space) to a
-// small host vector v of 2^k entries.
-// Products are formed in extended precision.
-void apply_small(std::vector<cl>& v, uint32_t k, const std::vector<uint32_t>& pos,
-                 const std::vector<cl>& f) {
+// v <- (f on local positions pos[0..m-1] of a k-bit space) v for a small host matrix v of 2^k x 2^k
+// entries (rows first).  Products are formed in extended precision; those with a zero of f, and
+// where every factor of a sum is still zero (`filled`: the columns of each row that need not be),
+// are left out: the columns start as unit vectors, and most gates have zeros and real entries.
+void apply_small(std::vector<cl>& v, std::vector<uint64_t>& filled, uint32_t k,
+                 const std::vector<uint32_t>& pos, const std::vector<cl>& f) {
     const uint32_t m = static_cast<uint32_t>(pos.size());
-    const uint64_t dim = uint64_t{1} << m;
+    const uint64_t dim = uint64_t{1} << m, cols = uint64_t{1} << k;
     std::vector<uint32_t> sorted = pos;
     std::sort(sorted.begin(), sorted.end());
     std::vector<uint64_t> off(dim, 0);
     for (uint64_t l = 0; l < dim; ++l)
         for (uint32_t j = 0; j < m; ++j)
             if ((l >> j) & 1) off[l] |= uint64_t{1} << pos[j];
-    const uint64_t groups = (uint64_t{1} << k) >> m;
-    std::vector<cl> a(dim);
+    const uint64_t groups = cols >> m;
+    const cl zero{0, 0};
+    std::vector<cl> a(dim * cols);
+    std::vector<uint64_t> from(dim);
+    const uint64_t every = cols >= 64 ? ~uint64_t{0} : (uint64_t{1} << cols) - 1;
     for (uint64_t g = 0; g < groups; ++g) {
         uint64_t base = g;
         for (uint32_t p : sorted) {
             const uint64_t low = (uint64_t{1} << p) - 1;
             base = ((base & ~low) << 1) | (base & low);
         }
-        for (uint64_t l = 0; l < dim; ++l) a[l] = v[base | off[l]];
+        for (uint64_t l = 0; l < dim; ++l) {
+            std::copy_n(v.data() + (base | off[l]) * cols, cols, a.data() + l * cols);
+            from[l] = cols > 64 ? every : filled[base | off[l]];
+        }
         for (uint64_t r = 0; r < dim; ++r) {
-            cl s{0.0, 0.0};
-            for (uint64_t c = 0; c < dim; ++c) s += wide_mul(f[r * dim + c], a[c]);
-            v[base | off[r]] = s;
+            cl* const s = v.data() + (base | off[r]) * cols;
+            uint64_t done = 0;
+            for (uint64_t c = 0; c < dim; ++c) {
+                const cl w = f[r * dim + c];
+                if (w == zero || from[c] == 0) continue;
+                const cl* const x = a.data() + c * cols;
+                const long double wr = w.real();
+                auto product = [&](uint64_t i) {
+                    return w.imag() == 0.0L ? cl{wr * x[i].real(), wr * x[i].imag()} : wide_mul(w, x[i]);
+                };
+                if (from[c] == every && done == every) {
+                    for (uint64_t i = 0; i < cols; ++i) s[i] += product(i);
+                } else if (from[c] == every && done == 0) {
+                    for (uint64_t i = 0; i < cols; ++i) s[i] = product(i);
+                } else {
+                    if (done == 0) std::fill_n(s, cols, zero);
+                    for (uint64_t b = from[c]; b; b &= b - 1) {
+                        const uint64_t i = static_cast<uint64_t>(__builtin_ctzll(b));
+                        s[i] += product(i);
+                    }
+                }
+                done |= from[c];
+            }
+            if (done == 0) std::fill_n(s, cols, zero);
+            filled[base | off[r]] = done;
         }
     }
 }
@@ -546,9 +575,11 @@ std::vector<cl> block_matrix_wide(const FusedBlock& b, const std::vector<GateDes
     const uint32_t k = static_cast<uint32_t>(b.qubits.size());
     const uint64_t dim = uint64_t{1} << k;
     std::vector<cl> m(dim * dim, cl{0, 0});
-    // columns evolve independently: column c starts as e_c
-    std::vector<std::vector<cl>> cols(dim, std::vector<cl>(dim, cl{0, 0}));
-    for (uint64_t c = 0; c < dim; ++c) cols[c][c] = 1.0L;
+    std::vector<uint64_t> filled(dim, 0);
+    for (uint64_t c = 0; c < dim; ++c) {
+        m[c * dim + c] = 1.0L;
+        if (c < 64) filled[c] = uint64_t{1} << c;
+    }
     for (uint32_t gi : b.gates) {
         const GateDesc& g = gates[gi];
         std::vector<uint32_t> pos;
@@ -562,10 +593,8 @@ std::vector<cl> block_matrix_wide(const FusedBlock& b, const std::vector<GateDes
         } else {
             for (const cd& z : g.full_matrix()) f.push_back(z);
         }
-        for (uint64_t c = 0; c < dim; ++c) apply_small(cols[c], k, pos, f);
+        apply_small(m, filled, k, pos, f);
     }
-    for (uint64_t c = 0; c < dim; ++c)
-        for (uint64_t r = 0; r < dim; ++r) m[r * dim + c] = cols[c][r];
     return m;
 }
 

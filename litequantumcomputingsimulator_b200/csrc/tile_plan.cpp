@@ -1203,40 +1203,25 @@ bool fits(const LocalOp& o, bool mma, const Lay& ly) {
 }
 
 // Scan of the pending ops under layout ly: every op that commutes with all skipped ops
-// before it and fits the layout is applied.  Returns the count; with `emitted` the applied
-// ops move there (in order) and `pending` keeps the rest.  mma[i]: op i is a tensor-path op.
-size_t scan(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
-            const std::vector<uint8_t>& mma, std::vector<uint32_t>& pending, const Lay& ly,
-            std::vector<uint32_t>* emitted, bool rot) {
+// before it and fits the layout is applied.  The applied ops move to `emitted` (in order) and
+// `pending` keeps the rest.  mma[i]: op i is a tensor-path op.
+void scan(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
+          const std::vector<uint8_t>& mma, std::vector<uint32_t>& pending, const Lay& ly,
+          std::vector<uint32_t>& emitted) {
     uint32_t busy_nd = 0, busy_dg = 0;
-    size_t cnt = 0;
     std::vector<uint32_t> rest;
     for (uint32_t i : pending) {
         const Use& u = use[i];
         const bool blocked = (u.nd & (busy_nd | busy_dg)) != 0 || (u.dg & busy_nd) != 0;
         if (!blocked && fits(ops[i], mma[i] != 0, ly)) {
-            if (!rot || off_diagonal(ops[i])) ++cnt;   // rotation form: diagonals cost no layout
-            if (emitted) emitted->push_back(i);
+            emitted.push_back(i);
         } else {
             busy_nd |= u.nd;
             busy_dg |= u.dg;
-            if (emitted) rest.push_back(i);
+            rest.push_back(i);
         }
     }
-    if (emitted) pending = std::move(rest);
-    return cnt;
-}
-
-// Register-path dense ops of `pending` whose targets all lie in S (a tie-break: later use
-// of a layout).
-size_t covered(const std::vector<LocalOp>& ops, const std::vector<uint8_t>& mma,
-               const std::vector<uint32_t>& pending, uint32_t S) {
-    size_t c = 0;
-    for (uint32_t i : pending)
-        if (off_diagonal(ops[i]) && !mma[i] &&
-            (target_mask(ops[i]) & ~S) == 0)
-            ++c;
-    return c;
+    pending = std::move(rest);
 }
 
 // Layout of register set S, warp bits W and lane pair P on an m-bit tile.  Thread-index bits
@@ -1335,35 +1320,96 @@ uint32_t pick_warp_bits(const std::vector<LocalOp>& ops, const std::vector<uint3
     return W;
 }
 
-// Register sets of size kRegBits inside `allowed` that contain `must`, best first by
-// (ops applied now with warp bits W and lane pair P, register-path dense ops covered later,
-// usable as the final layout, and — when the warp bits are known, `lane_pool` being the
-// tile bits outside them — lanes that take all three residues mod 3, which keeps the remaps
-// free of bank conflicts).
+// The register set of size kRegBits inside `allowed` that contains `must` and is best by
+// (ops applied now with warp bits W and lane pair P, register-path dense ops covered later — a
+// tie-break: later use of a layout —, usable as the final layout, and — when the warp bits are
+// known, `lane_pool` being the tile bits outside them — lanes that take all three residues mod 3,
+// which keeps the remaps free of bank conflicts).  The first of equals in ascending order.
+// Most of the time of planning a new circuit goes into these scans, so they run over masks
+// alone, from one table per call, and end where every tile bit is blocked.
 uint32_t choose_set(const std::vector<LocalOp>& ops, const std::vector<Use>& use,
-                    const std::vector<uint8_t>& mma, std::vector<uint32_t>& pending,
+                    const std::vector<uint8_t>& mma, const std::vector<uint32_t>& pending,
                     uint32_t must, uint32_t allowed, uint32_t m, bool rot, uint32_t lane_pool = 0,
                     uint32_t P = 0, uint32_t W = 0) {
+    struct Row {
+        uint32_t nd, dg;   // Use
+        uint32_t need;     // bits that must be register bits (all ones: it never fits)
+        uint32_t counts;   // rotation form: diagonals cost no layout
+    };
+    std::vector<Row> rows;
+    rows.reserve(pending.size());
+    uint32_t single[32] = {};              // register-path dense ops by target, and the targets of
+    std::vector<uint32_t> several;         // those with more than one
+    for (uint32_t i : pending) {
+        const LocalOp& o = ops[i];
+        const uint32_t t = target_mask(o);
+        const bool off = off_diagonal(o);
+        // fits(), for the part that does not depend on the set
+        uint32_t need = 0;
+        if (o.kind == kTilePauli) need = (t & W) == 0 ? 0u : ~0u;
+        else if (o.kind == kTileRot) need = t;
+        else if (o.kind == kTileDense && !mma[i]) need = t;
+        else if (o.kind == kTileDense) need = P != 0 && (t & ~P) == 0 ? o.lmask & ~W : ~0u;
+        rows.push_back({use[i].nd, use[i].dg, need, !rot || off ? 1u : 0u});
+        if (!off || mma[i]) continue;
+        if (o.lt.size() == 1) ++single[o.lt[0]];
+        else several.push_back(t);
+    }
     uint32_t best = 0;
     size_t best_now = 0, best_later = 0;
     bool best_final = false, best_spread = false, have = false;
-    const uint32_t lanes = (1u << kLaneBits) - 1u;
-    for (uint32_t S = 0; S < (1u << m); ++S) {
-        if (__builtin_popcount(S) != static_cast<int>(kRegBits) || (S & must) != must ||
-            (S & ~allowed) != 0)
-            continue;
-        const size_t now = scan(ops, use, mma, pending, Lay{S, W, P}, nullptr, rot);
-        const size_t later = covered(ops, mma, pending, S);
-        const bool fin = (S & lanes) == 0;
-        const bool spread = lane_pool != 0 && residues_spread(lane_pool & ~S);
-        const auto key = std::make_tuple(now, later, fin, spread);
-        if (!have || key > std::make_tuple(best_now, best_later, best_final, best_spread)) {
-            have = true;
-            best = S;
-            best_now = now;
-            best_later = later;
-            best_final = fin;
-            best_spread = spread;
+    const uint32_t lanes = (1u << kLaneBits) - 1u, all = (1u << m) - 1u;
+    // every set: `must` and `more` of the `free` bits, ascending (the next number with as many ones)
+    std::vector<uint32_t> sets;
+    const uint32_t free = allowed & ~must & all;
+    const int n_free = __builtin_popcount(free), more = static_cast<int>(kRegBits) - __builtin_popcount(must);
+    if (more < 0 || more > n_free) return 0;
+    for (uint32_t pick = (1u << more) - 1u; pick < (1u << n_free);) {
+        uint32_t S = must;
+        for (uint32_t f = free, x = pick; x; f &= f - 1, x >>= 1)
+            if (x & 1u) S |= f & (~f + 1u);
+        sets.push_back(S);
+        if (pick == 0) break;   // `must` alone
+        const uint32_t low = pick & (~pick + 1u), up = pick + low;
+        pick = up | (((pick ^ up) / low) >> 2);
+    }
+    constexpr size_t kLanes = 16;   // sets scanned side by side (vector instructions)
+    for (size_t s0 = 0; s0 < sets.size(); s0 += kLanes) {
+        const size_t n_sets = std::min(kLanes, sets.size() - s0);
+        uint32_t S[kLanes] = {}, busy_nd[kLanes] = {}, busy_dg[kLanes] = {}, now[kLanes] = {};
+        std::copy_n(sets.begin() + static_cast<long>(s0), n_sets, S);
+        for (size_t i = 0; i < rows.size(); ++i) {
+            const Row r = rows[i];
+            for (size_t l = 0; l < kLanes; ++l) {
+                const uint32_t clash = (r.nd & (busy_nd[l] | busy_dg[l])) | (r.dg & busy_nd[l]) | (r.need & ~S[l]);
+                const uint32_t waits = clash != 0 ? ~0u : 0u;
+                now[l] += r.counts & ~waits;
+                busy_nd[l] |= r.nd & waits;
+                busy_dg[l] |= r.dg & waits;
+            }
+            if (rot && i % 8 == 7) {   // (what touches no bit does not count there)
+                uint32_t blocked = all;
+                for (size_t l = 0; l < n_sets; ++l) blocked &= busy_nd[l];
+                if (blocked == all) break;
+            }
+        }
+        for (size_t l = 0; l < n_sets; ++l) {
+            if (have && now[l] < best_now) continue;
+            size_t later = 0;
+            for (uint32_t b = S[l]; b; b &= b - 1) later += single[__builtin_ctz(b)];
+            for (uint32_t t : several) later += (t & ~S[l]) == 0;
+            const bool fin = (S[l] & lanes) == 0;
+            const bool spread = lane_pool != 0 && residues_spread(lane_pool & ~S[l]);
+            const size_t count = now[l];
+            if (!have || std::make_tuple(count, later, fin, spread) >
+                             std::make_tuple(best_now, best_later, best_final, best_spread)) {
+                have = true;
+                best = S[l];
+                best_now = count;
+                best_later = later;
+                best_final = fin;
+                best_spread = spread;
+            }
         }
     }
     return best;
@@ -1757,11 +1803,12 @@ class DiagonalPool {
                     f = wide_mul(f, phase(*o));
                 }
             }
-            std::vector<cl> table(size, one);
+            cl table[1u << (kRegBits + kRegTableThreadBits)];
+            std::fill_n(table, size, one);
             for (uint32_t j = 0; j < k; ++j)
                 for (uint32_t x = 0; x < (1u << j); ++x) {
-                    table[x | (1u << j)] = wide_mul(table[x], bit[j][1]);
-                    table[x] = wide_mul(table[x], bit[j][0]);
+                    table[x | (1u << j)] = bit[j][1] == one ? table[x] : wide_mul(table[x], bit[j][1]);
+                    if (bit[j][0] != one) table[x] = wide_mul(table[x], bit[j][0]);
                 }
             for (const LocalOp* o : members) {
                 if (o->kind == kTilePhase) {
@@ -1786,13 +1833,12 @@ class DiagonalPool {
             const uint32_t flip = entry_mask(u & e.flipped);
             if (r.table == kRegTableExpanded) {
                 const uint32_t threads = 1u << width(u & ~S);
+                uint32_t offset[1u << kRegBits] = {};
+                for (uint32_t v = 1; v < (1u << kRegBits); ++v)
+                    offset[v] = offset[v & (v - 1)] + *reg_offset[__builtin_ctz(v)];
                 for (uint32_t t = 0; t < threads; ++t) {
-                    for (uint32_t v = 0; v < (1u << kRegBits); ++v) {
-                        uint32_t x = t;
-                        for (uint32_t i = 0; i < kRegBits; ++i)
-                            if ((v >> i) & 1) x += *reg_offset[i];
-                        e.mats.push_back(narrow(table[x ^ flip]));
-                    }
+                    for (uint32_t v = 0; v < (1u << kRegBits); ++v)
+                        e.mats.push_back(narrow(table[(t + offset[v]) ^ flip]));
                     e.mats.emplace_back(0.0, 0.0);
                 }
             } else {
@@ -2116,7 +2162,7 @@ bool lower_pass_reg_sel(const PlanItem& item, const std::vector<GateDesc>& gates
     bool sync_tiles = false;
     while (true) {
         std::vector<uint32_t> applied;
-        scan(ops, use, mma, pending, Lay{S, W, P}, &applied, rot);
+        scan(ops, use, mma, pending, Lay{S, W, P}, applied);
         for (uint32_t i : applied) seq.emplace_back(static_cast<int>(i), cur);
         if (pending.empty()) break;
         const LocalOp& f = ops[pending.front()];
