@@ -80,12 +80,16 @@ BlockPool<CudaBlocks>& blocks() {   // never destroyed: buffers may be freed dur
 void clear_buffer_pool(bool retire) { blocks().clear(retire); }
 
 void DeviceBuffer::release() {
+    if (ptr) release(bytes <= kBlockMax && CudaBlocks::wait(device, stream));
+}
+
+void DeviceBuffer::release(bool idle) {
     if (!ptr) return;
     void* p = ptr;
     const size_t b = bytes;
     ptr = nullptr;
     bytes = 0;
-    blocks().give(device, p, b, era, b <= kBlockMax && CudaBlocks::wait(device, stream));
+    blocks().give(device, p, b, era, idle);
 }
 
 void DeviceBuffer::ensure(size_t b) {
@@ -658,7 +662,7 @@ Program compile(const std::vector<GateDesc>& gates, uint32_t n, const FusionConf
 
 // ------------------------------------------------------------------ state handle
 
-lqcs_state::~lqcs_state() { lqcs_b200::pool_return(*this); }
+lqcs_state::~lqcs_state() { lqcs_b200::release_state(*this); }
 
 double* lqcs_state::partials(size_t values) {
     const size_t need = (lqcs_b200::kMaxReduceBlocks + 1) * values * 2 * sizeof(double) + 4096;
@@ -741,12 +745,10 @@ void clear_state_pool() {
     for (const PooledBuffer& b : drop) blocks().give(b.device, b.ptr, b.bytes, b.era, false);
 }
 
-void pool_return(lqcs_state& st) {
-    // (smaller ones are the block pool's)
-    if (!st.amps.ptr || st.amps.bytes <= kBlockMax || st.amps.bytes > kPoolMaxBytes) return;
+// The amplitude buffer goes to the kept ones (smaller buffers are the block pool's).
+static void keep_amplitudes(lqcs_state& st) {
+    if (st.amps.bytes <= kBlockMax || st.amps.bytes > kPoolMaxBytes) return;
     if (st.amps.era != blocks().era()) return;   // allocated before lqcs_release_caches: not kept
-    // the buffer is reused only after this state's work on it has finished
-    if (!CudaBlocks::wait(st.device, st.stream)) return;
     PooledBuffer evict{};
     {
         std::lock_guard<std::mutex> lk(pool_mu());
@@ -759,6 +761,14 @@ void pool_return(lqcs_state& st) {
     st.amps.ptr = nullptr;
     st.amps.bytes = 0;
     if (evict.ptr) blocks().give(evict.device, evict.ptr, evict.bytes, evict.era, false);
+}
+
+void release_state(lqcs_state& st) {
+    if (!st.amps.ptr && !st.scratch.ptr && !st.sample_scratch.ptr) return;
+    // the buffers are reused only after this state's work on them has finished
+    const bool idle = CudaBlocks::wait(st.device, st.stream);
+    if (idle && st.amps.ptr) keep_amplitudes(st);
+    for (DeviceBuffer* b : {&st.amps, &st.scratch, &st.sample_scratch}) b->release(idle);
 }
 
 std::unique_ptr<lqcs_state> new_state(uint32_t n, uint32_t batch, cudaStream_t stream) {

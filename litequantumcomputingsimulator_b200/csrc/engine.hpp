@@ -52,6 +52,7 @@ struct DeviceBuffer {
     }
     ~DeviceBuffer() { release(); }
     void release();
+    void release(bool idle);   // idle: the caller has waited for `stream`
     void ensure(size_t b);
     template <class T> T* as() const { return static_cast<T*>(ptr); }
 };
@@ -134,8 +135,9 @@ void clear_buffer_pool(bool retire = false);
 // The compiled program of a gate list: one of the last few circuits' or a new one.
 std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
                                               const FusionConfig& fc, cudaStream_t stream);
-// Called by ~lqcs_state: keeps a small amplitude buffer for the next state of its size.
-void pool_return(lqcs_state& st);
+// Called by ~lqcs_state: waits for the state's stream once and releases its buffers; an amplitude
+// buffer of 32 MiB to 1 GiB is kept for the next state of its size.
+void release_state(lqcs_state& st);
 
 // Compile a list of unitary gates to a Program (fused or gate by gate).
 Program compile(const std::vector<GateDesc>& gates, uint32_t n, const FusionConfig& fc,
