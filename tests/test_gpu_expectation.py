@@ -64,3 +64,19 @@ def test_many_terms_in_bounded_memory(n, letters):
     want = np.concatenate([A.expectation_terms(sv, [paulis[k] for k in some[i:i + 50]])
                            for i in range(0, len(some), 50)])
     assert np.max(np.abs(got[some] - want)) < 1e-12
+
+
+@pytest.mark.parametrize("n", [11, 12, 13, 15])
+def test_hamiltonian_apply_over_tiles(n):
+    """lambda = H psi on tiles of 2^12 amplitudes: one tile (to 12 qubits), and 2 and 8 tiles whose terms
+    have X masks above the tile (several groups).  <psi|H|psi> of the adjoint against the sum of the
+    terms' expectations; tolerance 1e-12 of the coefficients' sum."""
+    rng = np.random.default_rng(n)
+    ham = [(float(rng.normal()), "".join("IXYZ"[int(v)] for v in rng.integers(0, 4, n))) for _ in range(60)]
+    pc, _ = W.random_pauli_ansatz(n, 20, n)
+    params = W.random_parameter_sets(20, 3, n + 1)
+    got = A.batched_energy(ham, pc, params)
+    for e, p in zip(got, params):
+        sv = lq.Statevector(n).apply(pc.bind(p))
+        want = sum(c * v for (c, _s), v in zip(ham, A.expectation_terms(sv, [s for _c, s in ham])))
+        assert abs(e - want) < 1e-12 * sum(abs(c) for c, _s in ham)
