@@ -189,6 +189,9 @@ void Program::build(std::vector<DevOp> ops_in, cudaStream_t stream) {
         cuda_check(cudaMemcpyAsync(d_reg_ops.ptr, reg_ops.data(), reg_ops.size() * sizeof(RegOp),
                                    cudaMemcpyHostToDevice, stream),
                    "upload register pass records");
+    }
+    // (a pass may have no records: X gates alone negate bits at the store)
+    if (!reg_layouts.empty()) {
         d_reg_layouts.ensure(reg_layouts.size() * sizeof(RegLayout));
         cuda_check(cudaMemcpyAsync(d_reg_layouts.ptr, reg_layouts.data(),
                                    reg_layouts.size() * sizeof(RegLayout), cudaMemcpyHostToDevice,

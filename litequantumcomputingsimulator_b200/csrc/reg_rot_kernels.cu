@@ -19,6 +19,7 @@ void launch_rot_pass(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t bat
     RegPass p = pass;
     p.batch_stride = uint64_t{1} << n;
     p.n_tiles = (uint64_t{1} << n) >> p.m;
+    if (!d_layouts || !d_mats) throw std::logic_error("register tile pass: a table is not on the device");
     const size_t smem = reg_smem_bytes(p);
     if (smem > kTileMaxSmem || p.m < kRegMinBits || p.m > kRegMaxBits || p.h > kTileMaxHigh ||
         p.n_layouts < 1 || p.n_ops > kRegMaxRecords || p.n_mat > kRegMaxMatrix ||

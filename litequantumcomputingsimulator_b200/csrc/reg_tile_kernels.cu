@@ -591,6 +591,8 @@ void launch_reg_pass(const LaunchCtx& ctx, double2* st, uint32_t n, uint32_t bat
     p.batch_stride = uint64_t{1} << n;
     p.n_tiles = (uint64_t{1} << n) >> p.m;
     if (p.rot) throw std::logic_error("register tile pass: a pass in rotation form");
+    if (!d_layouts || (p.n_ops && !d_ops) || (p.n_mat && !d_mats))
+        throw std::logic_error("register tile pass: a table is not on the device");
     if (reg_pipe_enabled() && (p.m == 11 || p.m == 12)) {
         const size_t smem2 = reg_smem_bytes(p, 2);
         if (smem2 <= kRegPipeMaxSmem && p.n_ops <= kRegMaxRecords && p.n_mat <= kRegMaxMatrix &&
