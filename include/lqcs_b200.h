@@ -370,8 +370,8 @@ int lqcs_adjoint_gradient_multi(uint64_t n_problems, const lqcs_parametric_circu
 
 /* Frees what repeated calls keep on the device between calls — the resident state batches
  * and captured graphs of the last adjoint plans, the compiled programs of the last 16
- * circuits run (run / run_statevector reuse them for the same circuit and options) — and
- * the autotuner's choices.  Engine extension: no counterpart in the reference. */
+ * circuits run (run / run_statevector reuse them for the same circuit and options), the idle
+ * device buffers — and the autotuner's choices.  Buffers of live handles are freed with them.  Engine extension: no counterpart in the reference. */
 int lqcs_release_caches(void);
 
 /* Energies only, batched: the forward pass and <psi|H|psi> of lqcs_adjoint_gradient

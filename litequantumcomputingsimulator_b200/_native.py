@@ -112,6 +112,8 @@ class OpProfile(C.Structure):
     ]
 
 
+# (7: k_regrot on the default path; register passes of dense blocks — LQCS_REG_MMA, LQCS_REG_PIPE, or
+# a pass that has no rotation form — run k_regtile and are of the same kind)
 OP_KIND_NAMES = {0: "k_apply_1q", 1: "k_phase", 2: "k_dense", 3: "k_diag", 4: "k_perm",
                  5: "k_pauli", 6: "k_tile", 7: "k_regrot"}
 

@@ -142,7 +142,6 @@ void Program::build(std::vector<DevOp> ops_in, cudaStream_t stream) {
     mat_off.assign(ops.size(), 0);
     cyc_off.assign(ops.size(), 0);
     len_off.assign(ops.size(), 0);
-    source_gates = 0;
     for (size_t i = 0; i < ops.size(); ++i) {
         const DevOp& op = ops[i];
         source_gates += op.src_gates;
@@ -364,6 +363,8 @@ static Program assemble_tiles(const std::vector<GateDesc>& source, uint32_t n,
         }
         if (!part.gates.empty()) smem_pass(part);
     }
+    if (ops.empty())   // products that are the identity
+        for (const GateDesc& g : source) p.source_gates += g.is_unitary() ? 1 : 0;
     return p;
 }
 

@@ -64,3 +64,11 @@ def test_basis_states_run():
         assert np.all(lq.StatevectorSimulator(seed=1).run_registers(qc, 50) == want)
         noise = lq.NoiseModel().add_all_qubit_channel(lq.KrausChannel.phase_flip(0.3))
         assert np.all(lq.StatevectorSimulator(seed=1, noise=noise).run_registers(qc, 50) == want)
+
+
+@pytest.mark.parametrize("n", [12, 14])
+def test_gate_counts(n):
+    """Every source gate is counted, also where products of gates turn out to be the identity."""
+    for qc, gates in ((lq.QuantumCircuit(n).x(3).x(3), 2), (lq.QuantumCircuit(n).h(0).h(0).x(1), 3),
+                      (lq.QuantumCircuit(n).cx(0, 1).cx(0, 1).i(2), 3), (lq.QuantumCircuit(n), 0)):
+        assert CompiledCircuit(qc).n_gates == gates
