@@ -1831,18 +1831,19 @@ class DiagonalPool {
             r.nterm = static_cast<uint8_t>(gated.size());
             r.mat_off = static_cast<uint32_t>(e.mats.size());
             const uint32_t flip = entry_mask(u & e.flipped);
+            cd entry[1u << (kRegBits + kRegTableThreadBits)];
+            for (uint32_t x = 0; x < size; ++x) entry[x] = narrow(table[x ^ flip]);
             if (r.table == kRegTableExpanded) {
-                const uint32_t threads = 1u << width(u & ~S);
+                const uint32_t threads = 1u << width(u & ~S), row = (1u << kRegBits) + 1;
                 uint32_t offset[1u << kRegBits] = {};
                 for (uint32_t v = 1; v < (1u << kRegBits); ++v)
                     offset[v] = offset[v & (v - 1)] + *reg_offset[__builtin_ctz(v)];
-                for (uint32_t t = 0; t < threads; ++t) {
-                    for (uint32_t v = 0; v < (1u << kRegBits); ++v)
-                        e.mats.push_back(narrow(table[(t + offset[v]) ^ flip]));
-                    e.mats.emplace_back(0.0, 0.0);
-                }
+                e.mats.resize(e.mats.size() + threads * row);   // the row's last entry is not read
+                cd* out = e.mats.data() + r.mat_off;
+                for (uint32_t t = 0; t < threads; ++t, out += row)
+                    for (uint32_t v = 0; v < (1u << kRegBits); ++v) out[v] = entry[t + offset[v]];
             } else {
-                for (uint32_t x = 0; x < size; ++x) e.mats.push_back(narrow(table[x ^ flip]));
+                e.mats.insert(e.mats.end(), entry, entry + size);
             }
             for (const LocalOp* o : gated) {
                 const uint32_t em = entry_mask(o->lmask);
