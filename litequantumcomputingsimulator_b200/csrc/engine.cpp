@@ -181,9 +181,10 @@ void Program::build(std::vector<DevOp> ops_in, cudaStream_t stream) {
                                    cudaMemcpyHostToDevice, stream),
                    "upload tile matrices");
     }
-    std::vector<double2> rmats;
-    for (const cd& z : reg_mats) rmats.push_back(to_d2(z));
-    if (!reg_ops.empty()) {
+    // (the records of passes in rotation form are a kernel parameter)
+    const bool reads_ops = std::any_of(reg_passes.begin(), reg_passes.end(),
+                                       [](const RegPass& rp) { return !rp.rot; });
+    if (reads_ops && !reg_ops.empty()) {
         d_reg_ops.ensure(reg_ops.size() * sizeof(RegOp));
         cuda_check(cudaMemcpyAsync(d_reg_ops.ptr, reg_ops.data(), reg_ops.size() * sizeof(RegOp),
                                    cudaMemcpyHostToDevice, stream),
@@ -197,9 +198,10 @@ void Program::build(std::vector<DevOp> ops_in, cudaStream_t stream) {
                                    stream),
                    "upload register layouts");
     }
-    if (!rmats.empty()) {
-        d_reg_mats.ensure(rmats.size() * sizeof(double2));
-        cuda_check(cudaMemcpyAsync(d_reg_mats.ptr, rmats.data(), rmats.size() * sizeof(double2),
+    if (!reg_mats.empty()) {
+        static_assert(sizeof(cd) == sizeof(double2), "uploaded as they are");
+        d_reg_mats.ensure(reg_mats.size() * sizeof(double2));
+        cuda_check(cudaMemcpyAsync(d_reg_mats.ptr, reg_mats.data(), reg_mats.size() * sizeof(double2),
                                    cudaMemcpyHostToDevice, stream),
                    "upload register pass matrices");
     }

@@ -116,6 +116,7 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
     std::vector<Role> role(gates.size(), kOther);
     std::vector<std::vector<uint32_t>> on(n);   // gates touching each qubit, in order
     std::vector<uint32_t> at(gates.size(), 0);  // index of gate i in its target's list
+    std::vector<std::array<cd, 4>> base(gates.size());   // base matrix of one-qubit gates
     for (uint32_t i = 0; i < gates.size(); ++i) {
         const GateDesc& g = gates[i];
         if (g.type == LQCS_GATE_BARRIER) {
@@ -128,6 +129,7 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
                    g.type != LQCS_GATE_PERMUTATION) {
             if (g.base_qubits() == 1) {
                 const std::vector<cd> m = g.base_matrix();
+                std::copy_n(m.begin(), 4, base[i].begin());
                 if (g.n_controls == 0)
                     role[i] = m[1] == cd{0, 0} && m[2] == cd{0, 0} ? kDiag1 : kDense1;
                 else if (is_x_matrix(m) && g.qubits.size() <= 8)
@@ -160,7 +162,9 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
     struct Pending {
         M2 m{};
         uint32_t count = 0, src = 0;
-        GateDesc one;   // the gate itself while it is the only one
+        const GateDesc* one = nullptr;   // the source gate while it is the only one, or what a
+        int made = 0;                    // gate of this pass's own is made from (0: an H that is
+        double value = 0.0;              // rounded to `value`; RZ, P: their angle)
     };
     std::vector<Pending> pend(n);
     auto push = [&](GateDesc g) {
@@ -168,14 +172,14 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
         carry = 0;
         out.push_back(std::move(g));
     };
-    auto multiply = [&](uint32_t q, const GateDesc& g, uint32_t src) {
+    auto multiply = [&](uint32_t q, const M2& a, uint32_t src, const GateDesc* one, int made = 0,
+                        double value = 0.0) {
         Pending& p = pend[q];
-        std::vector<cl> a = g.wide;
-        if (a.empty())
-            for (const cd& z : g.base_matrix()) a.push_back(z);
         if (p.count == 0) {
-            p.m = {a[0], a[1], a[2], a[3]};
-            p.one = g;
+            p.m = a;
+            p.one = one;
+            p.made = made;
+            p.value = value;
         } else {
             const M2 b = p.m;
             p.m = {wide_mul(a[0], b[0]) + wide_mul(a[1], b[2]),
@@ -195,11 +199,16 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
             carry += p.src;   // such as the H H between two exchanged X
         } else {
             GateDesc g;
-            if (p.count == 1) {
-                g = std::move(p.one);
+            if (p.count == 1 && p.one) {
+                g = *p.one;
+            } else if (p.count == 1 && p.made) {
+                g = simple_gate(p.made, {q}, 0, {p.value});
+                g.wide.assign(p.m.begin(), p.m.end());
             } else {
                 g = simple_gate(LQCS_GATE_UNITARY, {q}, 0);
-                for (const cl& z : p.m) g.mat.push_back(narrow(z));
+                if (p.count == 1) g.mat = {p.value, p.value, p.value, -p.value};
+                else
+                    for (const cl& z : p.m) g.mat.push_back(narrow(z));
                 g.wide.assign(p.m.begin(), p.m.end());
             }
             g.src = p.src;
@@ -207,6 +216,15 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
         }
         p = Pending{};
     };
+    auto matrix_of = [&](uint32_t i) {
+        M2 a;
+        for (int e = 0; e < 4; ++e) a[e] = gates[i].wide.empty() ? cl{base[i][e]} : gates[i].wide[e];
+        return a;
+    };
+    // 1/sqrt(2) rounded up and down (see below)
+    const long double root = std::sqrt(0.5L);
+    const double nearest = static_cast<double>(root);
+    const double other = std::nextafter(nearest, nearest > root ? 0.0 : 1.0);
     for (uint32_t i = 0; i < gates.size(); ++i) {
         const GateDesc& g = gates[i];
         if (g.type == LQCS_GATE_BARRIER) {
@@ -216,14 +234,14 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
         }
         if (!g.slot && plain_1q(g)) {
             if (role[i] == kDiag1) {   // a damping factor: between two gates it would leave no
-                const std::vector<cd> m = g.base_matrix();   // rotation form, in a table it is free
+                const std::array<cd, 4>& m = base[i];   // rotation form, in a table it is free
                 if (std::abs(std::abs(m[0]) - std::abs(m[3])) > 1e-12) {
                     flush(g.qubits[0]);
                     push(g);
                     continue;
                 }
             }
-            multiply(g.qubits[0], g, g.src);
+            multiply(g.qubits[0], matrix_of(i), g.src, &g);
             continue;
         }
         if (role[i] == kCtrlX && (absorbs(i, -1) || absorbs(i, 1))) {
@@ -231,19 +249,13 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
             // The H before rounds 1/sqrt(2) up and the H after rounds it down: two of the same
             // would scale the state by 1 + 2e-16 for every exchanged X where they are folded
             // into dense blocks.
-            GateDesc h = simple_gate(LQCS_GATE_UNITARY, {t}, 0);
-            const long double r = std::sqrt(0.5L);
-            h.wide = {r, r, r, -r};
-            auto rounded = [&](double x) { h.mat = {x, x, x, -x}; };
-            const double nearest = static_cast<double>(r);
-            rounded(nearest);
-            multiply(t, h, 0);
+            const M2 h = {root, root, root, -root};
+            multiply(t, h, 0, nullptr, 0, nearest);
             for (uint32_t q : g.qubits) flush(q);
             GateDesc z = simple_gate(LQCS_GATE_Z, g.qubits, g.n_controls);
             z.src = g.src;
             push(std::move(z));
-            rounded(std::nextafter(nearest, nearest > r ? 0.0 : 1.0));
-            multiply(t, h, 0);
+            multiply(t, h, 0, nullptr, 0, other);
             continue;
         }
         if (g.type == LQCS_GATE_RZZ && g.n_controls == 0) {
@@ -253,22 +265,20 @@ std::vector<GateDesc> rotation_form(const std::vector<GateDesc>& gates, uint32_t
             const double th = g.params.at(0);
             const uint32_t rz = pend[b].count > 0 && pend[a].count == 0 ? b : a;
             const uint32_t ph = rz == a ? b : a;
-            GateDesc grz = simple_gate(LQCS_GATE_RZ, {rz}, 0, {th});
-            GateDesc gph = simple_gate(LQCS_GATE_P, {ph}, 0, {th});
             auto unit = [](long double x) { return cl{std::cos(x), std::sin(x)}; };
-            grz.wide = {unit(-0.5L * th), 0.0L, 0.0L, unit(0.5L * th)};
-            gph.wide = {1.0L, 0.0L, 0.0L, unit(th)};
+            const M2 grz = {unit(-0.5L * th), 0.0L, 0.0L, unit(0.5L * th)};
+            const M2 gph = {1.0L, 0.0L, 0.0L, unit(th)};
             const bool rz_now = pend[rz].count > 0, ph_now = pend[ph].count > 0;
-            if (rz_now) multiply(rz, grz, 0);
-            if (ph_now) multiply(ph, gph, 0);
+            if (rz_now) multiply(rz, grz, 0, nullptr, LQCS_GATE_RZ, th);
+            if (ph_now) multiply(ph, gph, 0, nullptr, LQCS_GATE_P, th);
             flush(a);
             flush(b);
             GateDesc cp = simple_gate(LQCS_GATE_P, {a, b}, 1, {-2.0 * th});
             cp.src = g.src;
             cp.wide = {1.0L, 0.0L, 0.0L, unit(-2.0L * th)};
             push(std::move(cp));
-            if (!rz_now) multiply(rz, grz, 0);
-            if (!ph_now) multiply(ph, gph, 0);
+            if (!rz_now) multiply(rz, grz, 0, nullptr, LQCS_GATE_RZ, th);
+            if (!ph_now) multiply(ph, gph, 0, nullptr, LQCS_GATE_P, th);
             continue;
         }
         for (uint32_t q : g.qubits) flush(q);
