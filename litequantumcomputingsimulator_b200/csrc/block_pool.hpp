@@ -209,7 +209,8 @@ class BlockPool {
         return drop;
     }
 
-    // Frees what is still the pool's (an address of an earlier era may be a later allocation's).
+    // Frees what is still the pool's (an address of an earlier era may be a later allocation's, of
+    // the pool or of others: such a free is tried once only).
     void release(const std::vector<Free>& drop) {
         for (const Free& f : drop) {
             {
@@ -220,6 +221,7 @@ class BlockPool {
             }
             if (Api::free(f.device, f.p)) continue;
             std::lock_guard<std::mutex> lk(mu_);
+            if (f.era != era_) continue;
             owned_.emplace(std::pair{f.device, f.p}, f.era);
             later_.push_back(f);
         }

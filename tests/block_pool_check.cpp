@@ -30,8 +30,9 @@ struct Fake {
     }
     static bool free(int, void* p) {
         if (refuse_free) return false;
-        if (held.erase(p) == 0) ++bad_frees;
-        return true;
+        if (held.erase(p) != 0) return true;
+        ++bad_frees;   // not an address of the device's
+        return false;
     }
 };
 using lqcs_b200::block_size;
@@ -147,14 +148,35 @@ void reset_device() {
     expect(big2 == big, "the fake device hands out the same addresses");
     pool.give(0, big, mib2, era, true);
     expect(Fake::held.count(big2) == 1, "a block of this era was freed as an old one");
+    expect(Fake::bad_frees == 0, "dead addresses were freed");
     expect(pool.take(0, mib2) != big2, "a block in use was handed out twice");
+}
+
+// Idle blocks from before a reset: their free fails, and is not tried again (their addresses may be
+// another library's by then).
+void reset_with_idle_blocks() {
+    Pool pool;
+    const size_t mib2 = size_t{2} << 20, mib4 = size_t{4} << 20;
+    void* a = pool.take(0, mib2);
+    void* b = pool.take(0, 1000);
+    pool.give(0, a, mib2, true);
+    pool.give(0, b, block_size(1000), true);
+    Fake::reset();
+    Fake::next += size_t{1} << 30;   // other addresses now
+    pool.clear(true);
+    expect(Fake::bad_frees == 2, "one try for each");
+    void* c = pool.take(0, mib4);
+    pool.give(0, c, mib4, true);
+    pool.clear();
+    pool.clear(true);
+    expect(Fake::bad_frees == 2 && Fake::held.empty(), "dead addresses were freed again");
 }
 
 }  // namespace
 
 int main() {
     for (auto* check : {pending_small, pending_slab_is_freed, pending_large, bounds, released_slab,
-                        released_large, reset_device}) {
+                        released_large, reset_device, reset_with_idle_blocks}) {
         Fake::reset();
         check();
     }
