@@ -859,6 +859,7 @@ std::string program_key(const std::vector<GateDesc>& gates, uint32_t n, const Fu
     put(&search, 1);
     put(&mma, 1);
     for (const GateDesc& g : gates) {
+        if (g.type == LQCS_GATE_MEASURE) continue;   // not part of the program
         const uint64_t sizes[5] = {g.qubits.size(), g.params.size(), g.mat.size(), g.perm.size(),
                                    g.pauli.size()};
         put(&g.type, sizeof g.type);
@@ -877,8 +878,14 @@ std::string program_key(const std::vector<GateDesc>& gates, uint32_t n, const Fu
 
 std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
                                               const FusionConfig& fc, cudaStream_t stream) {
-    if (fc.fuse && (fc.mode == kFuseLearned || fc.mode == kFuseAutotune))
-        return std::make_shared<const Program>(compile(gates, n, fc, stream));
+    auto compiled = [&] {
+        std::vector<GateDesc> keep;
+        keep.reserve(gates.size());
+        for (const GateDesc& g : gates)
+            if (g.type != LQCS_GATE_MEASURE) keep.push_back(g);
+        return std::make_shared<const Program>(compile(keep, n, fc, stream));
+    };
+    if (fc.fuse && (fc.mode == kFuseLearned || fc.mode == kFuseAutotune)) return compiled();
     const std::string key = program_key(gates, n, fc);
     {
         std::lock_guard<std::mutex> lk(prog_mu());
@@ -891,7 +898,7 @@ std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates
             }
         }
     }
-    auto prog = std::make_shared<const Program>(compile(gates, n, fc, stream));
+    auto prog = compiled();
     cuda_check(cudaStreamSynchronize(stream), "program upload");   // usable from any stream
     std::lock_guard<std::mutex> lk(prog_mu());
     progs().emplace_back(key, prog);
@@ -905,18 +912,14 @@ void clear_program_cache() {
 }
 
 void apply_circuit(lqcs_state& st, const std::vector<GateDesc>& gates, const FusionConfig& fc) {
-    std::vector<GateDesc> keep;
-    keep.reserve(gates.size());
     for (const GateDesc& g : gates) {
         if (g.type == LQCS_GATE_RESET)
             invalid("run_statevector: Reset is non-deterministic; use run() instead");
         if (g.type == LQCS_GATE_KRAUS)
             invalid("run_statevector: noisy simulation is stochastic (one trajectory is "
                     "not the quantum state); use run() or DensityMatrixSimulator");
-        if (g.type == LQCS_GATE_MEASURE) continue;
-        keep.push_back(g);
     }
-    const std::shared_ptr<const Program> p = cached_program(keep, st.n, fc, st.stream);
+    const std::shared_ptr<const Program> p = cached_program(gates, st.n, fc, st.stream);
     p->launch(st.ctx, st.d(), st.n, st.batch);
     st.sync();
 }

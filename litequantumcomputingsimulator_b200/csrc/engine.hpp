@@ -132,7 +132,8 @@ void clear_state_pool();
 // Free the idle blocks of the buffer pool; with `retire` what is in use leaves the pool too (each
 // block is freed when its buffer is, none is handed out again).
 void clear_buffer_pool(bool retire = false);
-// The compiled program of a gate list: one of the last few circuits' or a new one.
+// The compiled program of a gate list (without its Measures): one of the last few circuits' or a
+// new one.
 std::shared_ptr<const Program> cached_program(const std::vector<GateDesc>& gates, uint32_t n,
                                               const FusionConfig& fc, cudaStream_t stream);
 // Called by ~lqcs_state: waits for the state's stream once and releases its buffers; an amplitude
